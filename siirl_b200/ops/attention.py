@@ -15,8 +15,11 @@ from . import lib as _lib
 from . import reference as ref
 
 
+FWD_TILE = 256      # query rows of one block of the forward kernel
+
+
 class SeqInfo:
-    """Sequence boundaries of a packed batch plus the 128-row tile lists the attention kernels need."""
+    """Sequence boundaries of a packed batch plus the tile lists the attention kernels need."""
 
     def __init__(self, seqlens: Sequence[int], device=None):
         self.seqlens: List[int] = [int(x) for x in seqlens]
@@ -27,7 +30,7 @@ class SeqInfo:
         self.total = cu[-1]
         self.max_seqlen = max(self.seqlens) if self.seqlens else 0
         self.device = device
-        self._tiles = None
+        self._tiles = {}
         self._cu_dev = None
         self._pos = None
 
@@ -46,31 +49,25 @@ class SeqInfo:
             self._pos = pos.to(self.device) if self.device is not None else pos
         return self._pos
 
-    def tiles(self, q_start: Optional[Sequence[int]] = None):
-        """(seq_start, seq_len, offset) int32 device tensors, one entry per 128-row tile; longest
-        sequences' last tiles first so the heaviest causal tiles start early.  ``q_start[i]`` (a multiple of 128)
-        leaves out the query tiles of sequence i below that row: chunked prefill computes only the new rows."""
-        if q_start is not None:
-            start, length, off = [], [], []
-            for i, n in enumerate(self.seqlens):
-                for t0 in range(int(q_start[i]) // 128 * 128, n, 128):
-                    start.append(self.cu_seqlens_cpu[i])
-                    length.append(n)
-                    off.append(t0)
-            order = sorted(range(len(off)), key=lambda k: -off[k])
-            mk = lambda xs: torch.tensor([xs[k] for k in order], dtype=torch.int32, device=self.device)  # noqa: E731
-            return (mk(start), mk(length), mk(off), len(off))
-        if self._tiles is None:
-            start, length, off = [], [], []
-            for i, n in enumerate(self.seqlens):
-                for t0 in range(0, n, 128):
-                    start.append(self.cu_seqlens_cpu[i])
-                    length.append(n)
-                    off.append(t0)
-            order = sorted(range(len(off)), key=lambda k: -off[k])
-            mk = lambda xs: torch.tensor([xs[k] for k in order], dtype=torch.int32, device=self.device)  # noqa: E731
-            self._tiles = (mk(start), mk(length), mk(off), len(off))
-        return self._tiles
+    def tiles(self, q_start: Optional[Sequence[int]] = None, rows: int = 128):
+        """(seq_start, seq_len, offset) int32 device tensors, one entry per tile of ``rows`` rows (the backward kernel
+        takes 128, the forward kernel 256); longest sequences' last tiles first so the heaviest causal tiles start
+        early.  ``q_start[i]`` leaves out the rows of sequence i below ``q_start[i] // 128 * 128``: chunked prefill
+        computes only the new rows."""
+        if q_start is None and rows in self._tiles:
+            return self._tiles[rows]
+        start, length, off = [], [], []
+        for i, n in enumerate(self.seqlens):
+            for t0 in range(int(q_start[i]) // 128 * 128 if q_start is not None else 0, n, rows):
+                start.append(self.cu_seqlens_cpu[i])
+                length.append(n)
+                off.append(t0)
+        order = sorted(range(len(off)), key=lambda k: -off[k])
+        mk = lambda xs: torch.tensor([xs[k] for k in order], dtype=torch.int32, device=self.device)  # noqa: E731
+        tiles = (mk(start), mk(length), mk(off), len(off))
+        if q_start is None:
+            self._tiles[rows] = tiles
+        return tiles
 
 
 class _AttnFn(torch.autograd.Function):
@@ -80,7 +77,7 @@ class _AttnFn(torch.autograd.Function):
         T = qkv.shape[0]
         out = torch.empty(T, hq * d, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-        ts, tl, t0, n = info.tiles(q_start)
+        ts, tl, t0, n = info.tiles(q_start, FWD_TILE)
         rc = L.sb_fmha_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T,
                            hq, hkv, d, int(causal), ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)),
                            _lib.stream())

@@ -30,7 +30,7 @@ import torch
 import torch.distributed as dist
 
 from ..ops import lib as _lib
-from ..ops.attention import SeqInfo
+from ..ops.attention import FWD_TILE, SeqInfo
 from .ulysses import _PullBlock
 
 
@@ -65,7 +65,7 @@ def _block_fwd(qkv, info: SeqInfo, hq, hkv, d, causal, scale) -> Tuple[torch.Ten
     L = _lib.get_lib()
     out = torch.empty(T, hq * d, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-    ts, tl, t0, n = info.tiles()
+    ts, tl, t0, n = info.tiles(rows=FWD_TILE)
     _lib.check(L.sb_fmha_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n,
                              T, hq, hkv, d, int(causal), ctypes.c_float(scale),
                              _lib.ptr(_lib.status_word(qkv.device)), _lib.stream()), "sb_fmha_fwd")

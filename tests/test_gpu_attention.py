@@ -61,3 +61,25 @@ def test_attention_fwd_bwd(cfg, causal):
     # per-row check: no single token's gradient is off
     row_err = (qkv.grad.float() - xr.grad).norm(dim=1) / (xr.grad.norm(dim=1) + 1e-3)
     assert row_err.max().item() < 0.1, row_err.argmax().item()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("d,hq,hkv,scale,gain", [(128, 4, 2, None, 0.5), (64, 7, 1, None, 0.5), (128, 2, 2, -0.11, 0.5),
+                                                 (64, 2, 1, 0.0, 0.5), (128, 2, 1, None, 4.0), (64, 2, 2, None, 4.0)])
+def test_attention_fwd_tiles(d, hq, hkv, scale, gain, causal):
+    """Sequences around the tile sizes (128 keys, 256 rows), more key tiles than the ring has stages, scales of either
+    sign, and scores so far apart that the running maximum moves by more than the lazy bound."""
+    seqlens = [1, 127, 128, 129, 255, 256, 257, 385, 1500, 2]
+    torch.manual_seed(1)
+    T = sum(seqlens)
+    scale = scale if scale is not None else 1.0 / math.sqrt(d)
+    qkv = (gain * torch.randn(T, (hq + 2 * hkv) * d, device=DEV)).to(torch.bfloat16)
+    out = attention_packed(qkv, SeqInfo(seqlens, device=DEV), hq, hkv, d, causal=causal, scale=scale)
+    lib.check_status()
+    q, k, v = qkv.float().split([hq * d, hkv * d, hkv * d], dim=-1)
+    want = ref.attention_varlen(q.reshape(T, hq, d), k.reshape(T, hkv, d), v.reshape(T, hkv, d),
+                                torch.tensor([0] + list(torch.tensor(seqlens).cumsum(0))), causal=causal,
+                                scale=scale).reshape(T, hq * d)
+    # weights and outputs are rounded to bf16 (2^-9 each, relative): 1e-2 of a row leaves a factor of two and a half
+    row_err = (out.float() - want).norm(dim=1) / want.norm(dim=1)
+    assert row_err.max().item() < 1e-2, row_err.argmax().item()

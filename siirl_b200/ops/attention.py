@@ -16,6 +16,7 @@ from . import reference as ref
 
 
 FWD_TILE = 256      # query rows of one block of the forward kernel
+_NUM_SMS = 148
 
 
 class SeqInfo:
@@ -50,24 +51,61 @@ class SeqInfo:
         return self._pos
 
     def tiles(self, q_start: Optional[Sequence[int]] = None, rows: int = 128):
-        """(seq_start, seq_len, offset) int32 device tensors, one entry per tile of ``rows`` rows (the backward kernel
-        takes 128, the forward kernel 256); longest sequences' last tiles first so the heaviest causal tiles start
-        early.  ``q_start[i]`` leaves out the rows of sequence i below ``q_start[i] // 128 * 128``: chunked prefill
+        """(seq_start, seq_len, offset) int32 device tensors, one entry per tile of ``rows`` query rows; longest
+        sequences' last tiles first so the heaviest causal tiles start early.  ``q_start[i]`` leaves out the rows of sequence i below ``q_start[i] // 128 * 128``: chunked prefill
         computes only the new rows."""
         if q_start is None and rows in self._tiles:
             return self._tiles[rows]
-        start, length, off = [], [], []
-        for i, n in enumerate(self.seqlens):
-            for t0 in range(int(q_start[i]) // 128 * 128 if q_start is not None else 0, n, rows):
-                start.append(self.cu_seqlens_cpu[i])
-                length.append(n)
-                off.append(t0)
-        order = sorted(range(len(off)), key=lambda k: -off[k])
-        mk = lambda xs: torch.tensor([xs[k] for k in order], dtype=torch.int32, device=self.device)  # noqa: E731
-        tiles = (mk(start), mk(length), mk(off), len(off))
+        entries = [(self.cu_seqlens_cpu[i], n, t0) for i, n in enumerate(self.seqlens)
+                   for t0 in range(int(q_start[i]) // 128 * 128 if q_start is not None else 0, n, rows)]
+        tiles = self._device_tiles(sorted(entries, key=lambda e: -e[2]))
         if q_start is None:
             self._tiles[rows] = tiles
         return tiles
+
+    def kv_tiles(self):
+        """The same for the 128-row K/V tiles of the backward kernel: a causal tile meets the query rows from its own
+        on, so the tiles with most rows behind them come first."""
+        if "kv" not in self._tiles:
+            entries = [(self.cu_seqlens_cpu[i], n, t0) for i, n in enumerate(self.seqlens) for t0 in range(0, n, 128)]
+            self._tiles["kv"] = self._device_tiles(sorted(entries, key=lambda e: e[2] - e[1]))
+        return self._tiles["kv"]
+
+    def _device_tiles(self, entries):
+        mk = lambda k: torch.tensor([e[k] for e in entries], dtype=torch.int32, device=self.device)  # noqa: E731
+        return (mk(0), mk(1), mk(2), len(entries))
+
+
+def bwd_head_splits(seqlens: Sequence[int], hq: int, hkv: int, causal: bool) -> int:
+    """Blocks over which the backward kernel divides the q heads of a kv head.  Splitting adds fp32 sums of dK and dV and a
+    pass that converts them, so it is done only as far as the block with most steps would outlast an SM's average share:
+    (28 / 4 heads, 8 x 2048: share 0.54, whole 0.86 ms, halves 1.05; 14 / 2 heads, 1 x 9900: share 1.9, whole 1.21 ms,
+    thirds 0.72)."""
+    rep = hq // hkv
+    tiles = [(n + 127) // 128 for n in seqlens]
+    total = sum(t * (t + 1) // 2 if causal else t * t for t in tiles) * hq
+    longest = max(tiles, default=0)
+    for splits in range(1, rep):
+        if -(-rep // splits) * longest * _NUM_SMS <= total:
+            return splits
+    return rep
+
+
+def fmha_bwd(qkv, out, lse, dout, info: SeqInfo, hq: int, hkv: int, d: int, causal: bool, scale: float) -> torch.Tensor:
+    """Gradient of the packed ``qkv`` from the forward kernel's outputs."""
+    L = _lib.get_lib()
+    T = qkv.shape[0]
+    dqkv = torch.empty_like(qkv)
+    delta = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
+    dq_acc = torch.empty(T, hq * d, dtype=torch.float32, device=qkv.device)
+    splits = bwd_head_splits(info.seqlens, hq, hkv, causal)
+    dkv_acc = torch.empty(T, 2 * hkv * d, dtype=torch.float32, device=qkv.device) if splits > 1 else None
+    ts, tl, t0, n = info.kv_tiles()
+    rc = L.sb_fmha_bwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(delta), _lib.ptr(dq_acc),
+                       _lib.ptr(dkv_acc), _lib.ptr(dqkv), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T, hq, hkv, d,
+                       int(causal), splits, ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)), _lib.stream())
+    _lib.check(rc, "sb_fmha_bwd")
+    return dqkv
 
 
 class _AttnFn(torch.autograd.Function):
@@ -90,18 +128,7 @@ class _AttnFn(torch.autograd.Function):
     def backward(ctx, dout):
         qkv, out, lse = ctx.saved_tensors
         info, hq, hkv, d, causal, scale = ctx.meta
-        L = _lib.get_lib()
-        T = qkv.shape[0]
-        dout = dout.contiguous()
-        dqkv = torch.empty_like(qkv)
-        delta = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-        dq_acc = torch.empty(T, hq * d, dtype=torch.float32, device=qkv.device)
-        ts, tl, t0, n = info.tiles()
-        rc = L.sb_fmha_bwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(delta),
-                           _lib.ptr(dq_acc), _lib.ptr(dqkv), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T, hq, hkv,
-                           d, int(causal), ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)),
-                           _lib.stream())
-        _lib.check(rc, "sb_fmha_bwd")
+        dqkv = fmha_bwd(qkv, out, lse, dout.contiguous(), info, hq, hkv, d, causal, scale)
         return dqkv, None, None, None, None, None, None, None
 
 

@@ -30,7 +30,7 @@ import torch
 import torch.distributed as dist
 
 from ..ops import lib as _lib
-from ..ops.attention import FWD_TILE, SeqInfo
+from ..ops.attention import FWD_TILE, SeqInfo, fmha_bwd
 from .ulysses import _PullBlock
 
 
@@ -90,16 +90,7 @@ def _block_bwd(qkv, out, lse, dout, info: SeqInfo, hq, hkv, d, causal, scale) ->
             dv = dv.reshape(n, hkv, rep, d).sum(2)
             dqkv[a:b] = torch.cat([dq.reshape(n, -1), dk.reshape(n, -1), dv.reshape(n, -1)], -1).to(qkv.dtype)
         return dqkv
-    L = _lib.get_lib()
-    dqkv = torch.empty_like(qkv)
-    delta = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-    dq_acc = torch.empty(T, hq * d, dtype=torch.float32, device=qkv.device)
-    ts, tl, t0, n = info.tiles()
-    _lib.check(L.sb_fmha_bwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(delta),
-                             _lib.ptr(dq_acc), _lib.ptr(dqkv), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T, hq, hkv,
-                             d, int(causal), ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)),
-                             _lib.stream()), "sb_fmha_bwd")
-    return dqkv
+    return fmha_bwd(qkv, out, lse, dout, info, hq, hkv, d, causal, scale)
 
 
 class RingContext:

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from siirl_b200.ops import lib, reference as ref
-from siirl_b200.ops.attention import SeqInfo, attention_packed
+from siirl_b200.ops.attention import SeqInfo, attention_packed, bwd_head_splits
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -83,3 +83,30 @@ def test_attention_fwd_tiles(d, hq, hkv, scale, gain, causal):
     # weights and outputs are rounded to bf16 (2^-9 each, relative): 1e-2 of a row leaves a factor of two and a half
     row_err = (out.float() - want).norm(dim=1) / want.norm(dim=1)
     assert row_err.max().item() < 1e-2, row_err.argmax().item()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("d,hq,hkv,repeat,splits", [(128, 3, 1, 1, 3), (64, 4, 2, 1, 2), (128, 2, 1, 80, 1), (64, 6, 2, 80, 1)])
+def test_attention_bwd_tiles(d, hq, hkv, repeat, splits, causal):
+    """Sequences around the 128-row tiles with the heads of a group in one block and divided over several."""
+    seqlens = [1, 127, 128, 129, 257] * repeat + [385]
+    assert bwd_head_splits(seqlens, hq, hkv, causal) == splits
+    torch.manual_seed(2)
+    T, tail = sum(seqlens), sum(seqlens[-6:])
+    scale = 1.0 / math.sqrt(d)
+    qkv = (0.7 * torch.randn(T, (hq + 2 * hkv) * d, device=DEV)).to(torch.bfloat16).requires_grad_()
+    out = attention_packed(qkv, SeqInfo(seqlens, device=DEV), hq, hkv, d, causal=causal)
+    g = torch.randn_like(out)
+    out.backward(g)
+    lib.check_status()
+    x = qkv.detach()[-tail:].float().requires_grad_()       # the last sequences stand for all
+    q, k, v = x.split([hq * d, hkv * d, hkv * d], dim=-1)
+    want = ref.attention_varlen(q.reshape(tail, hq, d), k.reshape(tail, hkv, d), v.reshape(tail, hkv, d),
+                                torch.tensor([0] + list(torch.tensor(seqlens[-6:]).cumsum(0))), causal=causal,
+                                scale=scale).reshape(tail, hq * d)
+    want.backward(g[-tail:].float())
+    got = qkv.grad[-tail:].float()
+    for a, b in ((0, hq * d), (hq * d, (hq + hkv) * d), ((hq + hkv) * d, None)):
+        # P, dS and the results are rounded to bf16 (2^-9 each): 2.5e-3 measured over these sizes, four times that allowed
+        assert _rel(got[:, a:b], x.grad[:, a:b]) < 1e-2
+    assert torch.isfinite(qkv.grad.float()).all()

@@ -68,6 +68,19 @@ def test_engine_matches_naive_greedy_with_prefix_sharing(tiny):
     assert len(eng.generate([[3, 4]], SamplingParams(max_new_tokens=2))) == 1
 
 
+@pytest.mark.parametrize("budget,slots,rounds", [(8192, 16, 3), (6, 16, 3), (6, 4, 9)])
+def test_engine_prefills_before_it_decodes(tiny, budget, slots, rounds):
+    """Prompts that need several prefill batches share the decode steps, unless the slots run out first."""
+    eng = RolloutEngine(tiny, max_num_seqs=slots, max_model_len=64, sync_interval=2, max_num_batched_tokens=budget)
+    prompts = [[10 + i, 11, 12, 40 + i][:2 + i % 3] for i in range(10)]
+    outs = eng.generate(prompts, SamplingParams(temperature=0.0, max_new_tokens=7, ignore_eos=True))
+    assert eng.stats["decode_steps"] == 2 * rounds
+    for o in outs:
+        alone = RolloutEngine(tiny, max_num_seqs=8, max_model_len=64).generate(
+            [prompts[o.prompt_index]], SamplingParams(temperature=0.0, max_new_tokens=7, ignore_eos=True))
+        assert o.token_ids == alone[0].token_ids and o.finish_reason == "length"
+
+
 def test_engine_eos_and_continuous_batching(tiny):
     eng = RolloutEngine(tiny, max_num_seqs=8, max_model_len=128, sync_interval=2)
     prompts = [[10 + i, 11, 12] for i in range(10)]          # 10 requests x n=2 > 8 slots -> several admission rounds

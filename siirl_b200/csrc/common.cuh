@@ -435,6 +435,35 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, int a_mn, i
 }
 
 // ---------------------------------------------------------------------------------------
+// Programmatic dependent launch: a kernel started with launch_chained may become resident while the kernel before it in
+// the stream still runs, so that launch latency and set-up (barriers, TMEM, descriptors) overlap its tail.  Such a kernel
+//   * calls chain_sync() in every thread before it touches memory that another kernel writes or reads: it returns when
+//     the kernels before have completed;
+//   * calls it after its TMEM allocation: chain_sync() also lets the next kernel start, whose own allocation must not be
+//     able to come first (it would keep the columns while it waits for this kernel).
+// Reads of the previous kernel's results go through plain pointers: __restrict__ const ones may be loaded early.
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void chain_sync() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline int launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// ---------------------------------------------------------------------------------------
 // misc numerics
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

@@ -12,10 +12,11 @@
 
 namespace sb {
 
-__global__ void decode_prepare_kernel(const unsigned char* __restrict__ finished, const int* __restrict__ ctx_len,
-                                      const int* __restrict__ rope_delta, int* __restrict__ pos,
-                                      int* __restrict__ seq_ids, int* __restrict__ seq_lens,
-                                      int* __restrict__ rope_pos, int S) {
+__global__ void decode_prepare_kernel(const unsigned char* finished, const int* ctx_len,
+                                      const int* rope_delta, int* pos,
+                                      int* seq_ids, int* seq_lens,
+                                      int* rope_pos, int S) {
+  chain_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= S) return;
   const bool active = finished[i] == 0;
@@ -26,12 +27,13 @@ __global__ void decode_prepare_kernel(const unsigned char* __restrict__ finished
   rope_pos[i] = active ? max(c - rope_delta[i], 0) : 0;
 }
 
-__global__ void decode_commit_kernel(const long long* __restrict__ tok, const float* __restrict__ lp,
-                                     unsigned char* __restrict__ finished, unsigned char* __restrict__ hit_eos,
-                                     int* __restrict__ ctx_len, int* __restrict__ remaining,
-                                     int* __restrict__ gen_index, long long* __restrict__ last_token,
-                                     long long* __restrict__ tokens_out, float* __restrict__ logp_out,
-                                     long long* __restrict__ step_counter, int S, int R, long long eos) {
+__global__ void decode_commit_kernel(const long long* tok, const float* lp,
+                                     unsigned char* finished, unsigned char* hit_eos,
+                                     int* ctx_len, int* remaining,
+                                     int* gen_index, long long* last_token,
+                                     long long* tokens_out, float* logp_out,
+                                     long long* step_counter, int S, int R, long long eos) {
+  chain_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *step_counter += 1;     // the sampler of this step has run already (same stream)
   if (i >= S) return;
@@ -60,9 +62,8 @@ using namespace sb;
 extern "C" int sb_decode_prepare(const void* finished, const int* ctx_len, const int* rope_delta, int* pos,
                                  int* seq_ids, int* seq_lens, int* rope_pos, int S, cudaStream_t stream) {
   if (S <= 0) return 0;
-  decode_prepare_kernel<<<(S + 127) / 128, 128, 0, stream>>>(reinterpret_cast<const unsigned char*>(finished),
+  return launch_chained(decode_prepare_kernel, (S + 127) / 128, 128, 0, stream, reinterpret_cast<const unsigned char*>(finished),
                                                              ctx_len, rope_delta, pos, seq_ids, seq_lens, rope_pos, S);
-  return (int)cudaGetLastError();
 }
 
 // eos < 0: no end-of-sequence token (or it is ignored)
@@ -71,8 +72,7 @@ extern "C" int sb_decode_commit(const long long* tok, const float* lp, void* fin
                                 float* logp_out, long long* step_counter, int S, int R, long long eos,
                                 cudaStream_t stream) {
   if (S <= 0) return 0;
-  decode_commit_kernel<<<(S + 127) / 128, 128, 0, stream>>>(
+  return launch_chained(decode_commit_kernel, (S + 127) / 128, 128, 0, stream,
       tok, lp, reinterpret_cast<unsigned char*>(finished), reinterpret_cast<unsigned char*>(hit_eos), ctx_len,
       remaining, gen_index, last_token, tokens_out, logp_out, step_counter, S, R, eos);
-  return (int)cudaGetLastError();
 }

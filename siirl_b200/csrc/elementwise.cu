@@ -50,10 +50,10 @@ constexpr int kNormMaxChunks = 4;  // hidden <= 256 * 8 * 4 = 8192
 
 template <int CH>
 __global__ void __launch_bounds__(kNormThreads)
-rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
-                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                   __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd_out, int T, int H, float eps) {
+rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y,
+                   __nv_bfloat16* h_out, float* rstd_out, int T, int H, float eps) {
   __shared__ float red[32];
+  chain_sync();
   const int nvec = H / 8;
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     float hv[CH][8];
@@ -210,8 +210,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restri
 // ---------------------------------------------------------------------------------------
 // SwiGLU on a fused gate|up projection: gu is [T, 2*I] with gate in columns [0,I), up in [I,2I).
 // ---------------------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int T,
-                                  int I) {
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out, int T, int I) {
+  chain_sync();
   const int nvec = I / 8;
   const long long total = (long long)T * nvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -254,8 +254,9 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 // ---------------------------------------------------------------------------------------
 SB_BOUNDS_WORD_DEFINE(elementwise)
 
-__global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
-                                     __nv_bfloat16* __restrict__ out, int T, int H, int V) {
+__global__ void embedding_fwd_kernel(const long long* ids, const __nv_bfloat16* table, __nv_bfloat16* out, int T, int H,
+                                     int V) {
+  chain_sync();
   const int nvec = H / 8;
   const long long total = (long long)T * nvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -317,17 +318,16 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* residual, const void* w
   const int ch = (H / 8 + kNormThreads - 1) / kNormThreads;
   const int grid = T < num_sms() * 8 ? T : num_sms() * 8;
 #define SB_LAUNCH(CH)                                                                                     \
-  rmsnorm_fwd_kernel<CH><<<grid, kNormThreads, 0, stream>>>(                                              \
+  return launch_chained(rmsnorm_fwd_kernel<CH>, grid, kNormThreads, 0, stream,                            \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, \
       (__nv_bfloat16*)h_out, rstd, T, H, eps)
   switch (ch) {
-    case 1: SB_LAUNCH(1); break;
-    case 2: SB_LAUNCH(2); break;
-    case 3: SB_LAUNCH(3); break;
-    default: SB_LAUNCH(4); break;
+    case 1: SB_LAUNCH(1);
+    case 2: SB_LAUNCH(2);
+    case 3: SB_LAUNCH(3);
+    default: SB_LAUNCH(4);
   }
 #undef SB_LAUNCH
-  return (int)cudaGetLastError();
 }
 
 extern "C" int sb_rmsnorm_bwd_blocks(int T) {
@@ -370,9 +370,8 @@ extern "C" int sb_rope(void* qkv, const int* pos, const float* cos_tab, const fl
 extern "C" int sb_swiglu_fwd(const void* gu, void* out, int T, int I, cudaStream_t stream) {
   if (I % 8) return -3;
   if (T == 0) return 0;
-  swiglu_fwd_kernel<<<grid_for((long long)T * (I / 8), 256), 256, 0, stream>>>((const __nv_bfloat16*)gu,
-                                                                             (__nv_bfloat16*)out, T, I);
-  return (int)cudaGetLastError();
+  return launch_chained(swiglu_fwd_kernel, grid_for((long long)T * (I / 8), 256), 256, 0, stream,
+                        (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I);
 }
 
 extern "C" int sb_swiglu_bwd(const void* gu, const void* dout, void* dgu, int T, int I, cudaStream_t stream) {
@@ -387,9 +386,8 @@ extern "C" int sb_embedding_fwd(const long long* ids, const void* table, void* o
                                 cudaStream_t stream) {
   if (H % 8) return -3;
   if (T == 0) return 0;
-  embedding_fwd_kernel<<<grid_for((long long)T * (H / 8), 256), 256, 0, stream>>>(
-      ids, (const __nv_bfloat16*)table, (__nv_bfloat16*)out, T, H, V);
-  return (int)cudaGetLastError();
+  return launch_chained(embedding_fwd_kernel, grid_for((long long)T * (H / 8), 256), 256, 0, stream, ids,
+                        (const __nv_bfloat16*)table, (__nv_bfloat16*)out, T, H, V);
 }
 
 extern "C" int sb_embedding_bwd(const long long* ids, const void* dout, float* dtable, int T, int H, int V,

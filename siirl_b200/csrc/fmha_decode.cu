@@ -66,11 +66,11 @@ __global__ void kv_copy_blocks_kernel(__nv_bfloat16* __restrict__ cache, const i
 // rotated k and the v heads of every row to its cache slot -- one launch instead of clone + rope + append.
 // One thread handles 8 rotation pairs (i, i + D/2) of one head, or 16 contiguous v elements.
 // ---------------------------------------------------------------------------------------
-__global__ void rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, const int* __restrict__ rope_pos,
-                                      int pos_rows, int sec0, int sec1, const float* __restrict__ cos_tab,
-                                      const float* __restrict__ sin_tab, const int* __restrict__ seq_ids,
-                                      const int* __restrict__ cache_pos, const int* __restrict__ block_table,
-                                      int max_blocks, __nv_bfloat16* __restrict__ cache, int T, int Hq, int Hkv, int D) {
+__global__ void rope_kv_append_kernel(__nv_bfloat16* qkv, int row_stride, const int* rope_pos, int pos_rows, int sec0,
+                                      int sec1, const float* cos_tab, const float* sin_tab, const int* seq_ids,
+                                      const int* cache_pos, const int* block_table, int max_blocks, __nv_bfloat16* cache,
+                                      int T, int Hq, int Hkv, int D) {
+  chain_sync();
   const int half = D / 2;
   const int units_per_head = half / 8;                 // 8 pairs per thread
   const int heads = Hq + 2 * Hkv;
@@ -409,10 +409,9 @@ extern "C" int sb_rope_kv_append(void* qkv, int row_stride, const int* rope_pos,
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)num_sms() * 8;
   if (blocks > cap) blocks = cap;
-  rope_kv_append_kernel<<<(int)blocks, 256, 0, stream>>>((__nv_bfloat16*)qkv, row_stride, rope_pos, pos_rows, sec0,
-                                                         sec1, cos_tab, sin_tab, seq_ids, cache_pos, block_table,
-                                                         max_blocks, (__nv_bfloat16*)cache, T, Hq, Hkv, D);
-  return (int)cudaGetLastError();
+  return launch_chained(rope_kv_append_kernel, (unsigned)blocks, 256, 0, stream, (__nv_bfloat16*)qkv, row_stride, rope_pos,
+                        pos_rows, sec0, sec1, cos_tab, sin_tab, seq_ids, cache_pos, block_table, max_blocks,
+                        (__nv_bfloat16*)cache, T, Hq, Hkv, D);
 }
 
 extern "C" int sb_kv_copy_blocks(void* cache, const int* src, const int* dst, int n_pairs, long long block_elems,

@@ -166,6 +166,7 @@ fmha_decode_split_kernel(const __grid_constant__ CUtensorMap map_cache, const __
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 128;      // output accumulator b at tmem_o + b * 128
+  chain_sync();
 
   // (chunk, sequence, kv head, first tile, tile count) of the first valid work item at or after `idx`; false at the end
   auto find_item = [&](int& idx, int& c, int& b, int& g, int& t0, int& n, int& seq_tiles) -> bool {
@@ -668,6 +669,7 @@ fmha_decode_split_kernel(const __grid_constant__ CUtensorMap map_cache, const __
 // merges the chunk partials of sequences longer than one chunk; zero rows for empty slots
 template <int D, bool WIN>
 __global__ void fmha_decode_merge_kernel(SplitParams p) {
+  chain_sync();
   const int b = blockIdx.x, h = blockIdx.y;
   const int ctx = p.seq_lens[b];
   int n_tiles = (ctx + kSBlk - 1) / kSBlk;
@@ -714,11 +716,9 @@ static int launch_decode_split(const CUtensorMap& mc, const CUtensorMap& mv, con
   }
   const int items = p.max_chunks * p.B * p.Hkv;
   const int grid = items < num_sms() ? items : num_sms();
-  kernel<<<grid, 160, L::kTotal, stream>>>(mc, mv, mq, p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
-  fmha_decode_merge_kernel<D, (MODE > 0)><<<dim3(p.B, p.Hq), D, 0, stream>>>(p);
-  return (int)cudaGetLastError();
+  const int rc = launch_chained(kernel, grid, 160, L::kTotal, stream, mc, mv, mq, p);
+  if (rc) return rc;
+  return launch_chained(fmha_decode_merge_kernel<D, (MODE > 0)>, dim3(p.B, p.Hq), D, 0, stream, p);
 }
 
 }  // namespace sb

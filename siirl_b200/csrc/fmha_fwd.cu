@@ -87,18 +87,6 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(empty + kStages);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = (int)(blockIdx.x % p.Hq), tile = (int)(blockIdx.x / p.Hq);
-  const int seq_start = p.tile_seq_start[tile], seq_len = p.tile_seq_len[tile], q0 = p.tile_q0[tile];
-  const int kvh = h / (p.Hq / p.Hkv);
-  // key tiles that query tile w walks over
-  auto key_tiles = [&](int w) {
-    const int first = q0 + w * 128;
-    if (first >= seq_len) return 0;
-    return ((p.causal ? min(first + 128, seq_len) : seq_len) + KV - 1) / KV;
-  };
-  const int n0 = key_tiles(0), n1 = key_tiles(1);
-  const int n_max = max(n0, n1);
-
   if (tid == 0) {
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_kv);
@@ -114,6 +102,18 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_sync();
+  const int h = (int)(blockIdx.x % p.Hq), tile = (int)(blockIdx.x / p.Hq);
+  const int seq_start = p.tile_seq_start[tile], seq_len = p.tile_seq_len[tile], q0 = p.tile_q0[tile];
+  const int kvh = h / (p.Hq / p.Hkv);
+  // key tiles that query tile w walks over
+  auto key_tiles = [&](int w) {
+    const int first = q0 + w * 128;
+    if (first >= seq_len) return 0;
+    return ((p.causal ? min(first + 128, seq_len) : seq_len) + KV - 1) / KV;
+  };
+  const int n0 = key_tiles(0), n1 = key_tiles(1);
+  const int n_max = max(n0, n1);
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
@@ -328,8 +328,7 @@ static int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mkv, const FmhaF
   }
   const long long blocks = (long long)num_tiles * p.Hq;
   if (blocks > 0x7fffffffll) return -4;
-  kernel<<<(unsigned)blocks, 320, L::kTotal, stream>>>(mq, mkv, p);
-  return (int)cudaGetLastError();
+  return launch_chained(kernel, (unsigned)blocks, 320, L::kTotal, stream, mq, mkv, p);
 }
 
 }  // namespace sb

@@ -428,7 +428,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   const bool is_copier = (int)blockIdx.x < copiers;
   const int cta0 = (int)blockIdx.x - copiers;       // index among the GEMM CTAs
   const int nctas = (int)gridDim.x - copiers;
-  const int ag_epoch = p.ag ? p.ag->local[0] + 1 : 0;
   const int num_tiles = tiles_mn * p.k_splits;  // k_splits holds the group count when group_rows is set
   constexpr uint32_t kTmemCols = 2 * BN;  // 256 or 512 (power of two)
 
@@ -453,6 +452,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_sync();
+  const int ag_epoch = p.ag ? p.ag->local[0] + 1 : 0;
 
   if (is_copier) {
     ag_copier<BN, L::kBarrierOffset>(p, smem, full_bar, STAGES);
@@ -713,6 +714,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   cluster_sync();  // the partner's barriers are initialised before anything is signalled across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_sync();
 
   auto tile_of = [&](int tile, int& m0, int& n0, int& kb0, int& kb1, long long& c_off) {
     const int ks = tile / tiles_mn;
@@ -894,8 +896,7 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   }
   const int tiles = ((p.M + 255) / 256) * ((p.N + kPairBN - 1) / kPairBN) * p.k_splits;
   const int clusters = tiles < max_clusters ? tiles : max_clusters;
-  kernel<<<2 * clusters, 192, kPairSmemBytes, stream>>>(ma, mb, p);
-  return (int)cudaGetLastError();
+  return launch_chained(kernel, 2 * clusters, 192, kPairSmemBytes, stream, ma, mb, p);
 }
 
 static int dispatch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int a_mn, int b_mn, int epi,
@@ -994,8 +995,7 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   int grid = tiles < avail ? tiles : avail;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   grid += p.ag_copiers;
-  kernel<<<grid, 192, L::kTotalBytes, stream>>>(ma, mb, p);
-  return (int)cudaGetLastError();
+  return launch_chained(kernel, grid, 192, L::kTotalBytes, stream, ma, mb, p);
 }
 
 template <int BN, int STAGES>
@@ -1024,9 +1024,9 @@ static int dispatch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const Gem
 
 namespace sb {
 // out[m, n] = bf16(sum_s slabs[s, m, n] + bias[n]); one thread per 8 columns
-__global__ void splitk_reduce_kernel(const float* __restrict__ slabs, long long slab_stride, int splits,
-                                     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out,
-                                     long long ldo, int M, int N) {
+__global__ void splitk_reduce_kernel(const float* slabs, long long slab_stride, int splits, const __nv_bfloat16* bias,
+                                     __nv_bfloat16* out, long long ldo, int M, int N) {
+  chain_sync();
   const int nvec = N / 8;
   const long long total = (long long)M * nvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -1069,9 +1069,8 @@ extern "C" int sb_splitk_reduce(const float* slabs, long long slab_stride, int s
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)num_sms() * 8;
   if (blocks > cap) blocks = cap;
-  splitk_reduce_kernel<<<(int)blocks, 256, 0, stream>>>(slabs, slab_stride, splits, (const __nv_bfloat16*)bias,
-                                                       (__nv_bfloat16*)out, ldo, M, N);
-  return (int)cudaGetLastError();
+  return launch_chained(splitk_reduce_kernel, (unsigned)blocks, 256, 0, stream, slabs, slab_stride, splits,
+                        (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, ldo, M, N);
 }
 
 struct GroupArgs {

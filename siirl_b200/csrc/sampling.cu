@@ -60,11 +60,11 @@ constexpr int kSampleThreads = 512;
 // sample_logits: logits the token is drawn from (possibly truncated with -inf by top-k / top-p);
 // stat_logits: logits that define the reported log-probability (normally the untruncated ones).
 __global__ void __launch_bounds__(kSampleThreads)
-sample_kernel(const float* __restrict__ sample_logits, const float* __restrict__ stat_logits, long long ld,
-              float inv_temp, int greedy, unsigned long long seed, unsigned long long step_host,
-              const long long* __restrict__ step_dev, long long* __restrict__ tokens, float* __restrict__ logp, int V,
-              int chunk, ArgStat* __restrict__ partial) {
+sample_kernel(const float* sample_logits, const float* stat_logits, long long ld, float inv_temp, int greedy,
+              unsigned long long seed, unsigned long long step_host, const long long* step_dev, long long* tokens,
+              float* logp, int V, int chunk, ArgStat* partial) {
   __shared__ ArgStat red[32];
+  chain_sync();
   const int row = blockIdx.x;
   const int v_begin = blockIdx.y * chunk, v_end = min(V, v_begin + chunk);
   const unsigned long long step = step_host + (step_dev ? (unsigned long long)*step_dev : 0ull);
@@ -135,9 +135,9 @@ sample_kernel(const float* __restrict__ sample_logits, const float* __restrict__
 }
 
 // merges the per-chunk partial results of one row (one warp per row)
-__global__ void sample_merge_kernel(const ArgStat* __restrict__ partial, int splits, const float* __restrict__ stat_logits,
-                                    long long ld, float inv_temp, long long* __restrict__ tokens,
-                                    float* __restrict__ logp, int rows) {
+__global__ void sample_merge_kernel(const ArgStat* partial, int splits, const float* stat_logits, long long ld,
+                                    float inv_temp, long long* tokens, float* logp, int rows) {
+  chain_sync();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -172,16 +172,15 @@ extern "C" int sb_sample(const float* sample_logits, const float* stat_logits, l
   const float inv_temp = greedy ? 1.f : 1.f / temperature;
   const float* zt = stat_logits ? stat_logits : sample_logits;
   if (!workspace || splits <= 1) {
-    sample_kernel<<<rows, kSampleThreads, 0, stream>>>(sample_logits, zt, ld, inv_temp, greedy, seed, step, step_dev,
-                                                       tokens, logp, V, V, nullptr);
-    return (int)cudaGetLastError();
+    return launch_chained(sample_kernel, rows, kSampleThreads, 0, stream, sample_logits, zt, ld, inv_temp, greedy, seed,
+                          step, step_dev, tokens, logp, V, V, (ArgStat*)nullptr);
   }
   // vocabulary split over `splits` blocks per row (workspace: rows * splits * 16 bytes), then one merge warp per row
   const int chunk = ((V + splits - 1) / splits + 3) / 4 * 4;
   dim3 grid(rows, splits);
-  sample_kernel<<<grid, kSampleThreads, 0, stream>>>(sample_logits, zt, ld, inv_temp, greedy, seed, step, step_dev,
-                                                     tokens, logp, V, chunk, reinterpret_cast<ArgStat*>(workspace));
-  sample_merge_kernel<<<(rows + 3) / 4, 128, 0, stream>>>(reinterpret_cast<const ArgStat*>(workspace), splits, zt, ld,
-                                                          inv_temp, tokens, logp, rows);
-  return (int)cudaGetLastError();
+  const int rc = launch_chained(sample_kernel, grid, kSampleThreads, 0, stream, sample_logits, zt, ld, inv_temp, greedy,
+                                seed, step, step_dev, tokens, logp, V, chunk, reinterpret_cast<ArgStat*>(workspace));
+  if (rc) return rc;
+  return launch_chained(sample_merge_kernel, (rows + 3) / 4, 128, 0, stream, reinterpret_cast<const ArgStat*>(workspace),
+                        splits, zt, ld, inv_temp, tokens, logp, rows);
 }

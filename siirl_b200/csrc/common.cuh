@@ -485,6 +485,18 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return y;
 }
 
+// v = sum over `splits` slabs of the eight floats at p (16-byte aligned), slab_stride floats apart
+__device__ __forceinline__ void slab_sum8(const float* p, long long slab_stride, int splits, float (&v)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s, p += slab_stride) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+    v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+  }
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -44,14 +44,17 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // ---------------------------------------------------------------------------------------
 // RMSNorm forward:  h = x (+ residual);  y = h * rsqrt(mean(h^2) + eps) * w
+// x may also be the fp32 partial sums of a split contraction (`slabs`), added up here: a pass of their own over so few
+// rows costs a launch (2.9 us against some 0.3 us of memory time for 8 x 896) and a rounding.
 // ---------------------------------------------------------------------------------------
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxChunks = 4;  // hidden <= 256 * 8 * 4 = 8192
 
 template <int CH>
 __global__ void __launch_bounds__(kNormThreads)
-rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y,
-                   __nv_bfloat16* h_out, float* rstd_out, int T, int H, float eps) {
+rmsnorm_fwd_kernel(const __nv_bfloat16* x, const float* slabs, long long slab_stride, int splits,
+                   const __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* h_out,
+                   float* rstd_out, int T, int H, float eps) {
   __shared__ float red[32];
   chain_sync();
   const int nvec = H / 8;
@@ -62,8 +65,12 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, const 
     for (int c = 0; c < CH; ++c) {
       const int vi = threadIdx.x + c * kNormThreads;
       if (vi < nvec) {
-        uint4 xv = reinterpret_cast<const uint4*>(x + (size_t)row * H)[vi];
-        bf16x8_to_float(xv, hv[c]);
+        if (slabs) {
+          slab_sum8(slabs + (size_t)row * H + vi * 8, slab_stride, splits, hv[c]);
+        } else {
+          uint4 xv = reinterpret_cast<const uint4*>(x + (size_t)row * H)[vi];
+          bf16x8_to_float(xv, hv[c]);
+        }
         if (residual) {
           float rv[8];
           uint4 r4 = reinterpret_cast<const uint4*>(residual + (size_t)row * H)[vi];
@@ -226,6 +233,21 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out, i
   }
 }
 
+// the same of a split contraction's partial sums: fp32 slabs [T, 2*I]
+__global__ void swiglu_slabs_kernel(const float* slabs, long long slab_stride, int splits, __nv_bfloat16* out, int T, int I) {
+  chain_sync();
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= I / 8) return;
+  for (int t = blockIdx.y; t < T; t += gridDim.y) {
+    float g[8], u[8], o[8];
+    slab_sum8(slabs + (size_t)t * 2 * I + v * 8, slab_stride, splits, g);
+    slab_sum8(slabs + (size_t)t * 2 * I + I + v * 8, slab_stride, splits, u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = g[i] / (1.f + __expf(-g[i])) * u[i];
+    reinterpret_cast<uint4*>(out + (size_t)t * I)[v] = float_to_bf16x8(o);
+  }
+}
+
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
                                   __nv_bfloat16* __restrict__ dgu, int T, int I) {
   const int nvec = I / 8;
@@ -311,16 +333,16 @@ static inline int grid_for(long long work, int threads, int per_sm = 8) {
 
 using namespace sb;
 
-extern "C" int sb_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* h_out,
-                              float* rstd, int T, int H, float eps, cudaStream_t stream) {
+static int rmsnorm_fwd(const void* x, const float* slabs, long long slab_stride, int splits, const void* residual,
+                       const void* w, void* y, void* h_out, float* rstd, int T, int H, float eps, cudaStream_t stream) {
   if (H % 8 || H > kNormThreads * 8 * kNormMaxChunks) return -3;
   if (T == 0) return 0;
   const int ch = (H / 8 + kNormThreads - 1) / kNormThreads;
   const int grid = T < num_sms() * 8 ? T : num_sms() * 8;
 #define SB_LAUNCH(CH)                                                                                     \
   return launch_chained(rmsnorm_fwd_kernel<CH>, grid, kNormThreads, 0, stream,                            \
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, \
-      (__nv_bfloat16*)h_out, rstd, T, H, eps)
+      (const __nv_bfloat16*)x, slabs, slab_stride, splits, (const __nv_bfloat16*)residual,                  \
+      (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, T, H, eps)
   switch (ch) {
     case 1: SB_LAUNCH(1);
     case 2: SB_LAUNCH(2);
@@ -328,6 +350,18 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* residual, const void* w
     default: SB_LAUNCH(4);
   }
 #undef SB_LAUNCH
+}
+
+extern "C" int sb_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* h_out,
+                              float* rstd, int T, int H, float eps, cudaStream_t stream) {
+  return rmsnorm_fwd(x, nullptr, 0, 0, residual, w, y, h_out, rstd, T, H, eps, stream);
+}
+
+// x = sum of `splits` fp32 slabs [T, H], slab_stride floats apart
+extern "C" int sb_rmsnorm_slabs_fwd(const float* slabs, long long slab_stride, int splits, const void* residual,
+                                    const void* w, void* y, void* h_out, int T, int H, float eps, cudaStream_t stream) {
+  if (splits < 1 || slab_stride % 4) return -3;
+  return rmsnorm_fwd(nullptr, slabs, slab_stride, splits, residual, w, y, h_out, nullptr, T, H, eps, stream);
 }
 
 extern "C" int sb_rmsnorm_bwd_blocks(int T) {
@@ -372,6 +406,14 @@ extern "C" int sb_swiglu_fwd(const void* gu, void* out, int T, int I, cudaStream
   if (T == 0) return 0;
   return launch_chained(swiglu_fwd_kernel, grid_for((long long)T * (I / 8), 256), 256, 0, stream,
                         (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I);
+}
+
+extern "C" int sb_swiglu_slabs_fwd(const float* slabs, long long slab_stride, int splits, void* out, int T, int I,
+                                   cudaStream_t stream) {
+  if (I % 8 || splits < 1 || slab_stride % 4) return -3;
+  if (T == 0) return 0;
+  return launch_chained(swiglu_slabs_kernel, dim3((I / 8 + 127) / 128, T < 65535 ? T : 65535), 128, 0, stream, slabs,
+                        slab_stride, splits, (__nv_bfloat16*)out, T, I);
 }
 
 extern "C" int sb_swiglu_bwd(const void* gu, const void* dout, void* dgu, int T, int I, cudaStream_t stream) {

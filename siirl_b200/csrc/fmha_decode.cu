@@ -66,7 +66,8 @@ __global__ void kv_copy_blocks_kernel(__nv_bfloat16* __restrict__ cache, const i
 // rotated k and the v heads of every row to its cache slot -- one launch instead of clone + rope + append.
 // One thread handles 8 rotation pairs (i, i + D/2) of one head, or 16 contiguous v elements.
 // ---------------------------------------------------------------------------------------
-__global__ void rope_kv_append_kernel(__nv_bfloat16* qkv, int row_stride, const int* rope_pos, int pos_rows, int sec0,
+__global__ void rope_kv_append_kernel(__nv_bfloat16* qkv, int row_stride, const float* slabs, long long slab_stride,
+                                      int splits, const __nv_bfloat16* bias, const int* rope_pos, int pos_rows, int sec0,
                                       int sec1, const float* cos_tab, const float* sin_tab, const int* seq_ids,
                                       const int* cache_pos, const int* block_table, int max_blocks, __nv_bfloat16* cache,
                                       int T, int Hq, int Hkv, int D) {
@@ -82,13 +83,35 @@ __global__ void rope_kv_append_kernel(__nv_bfloat16* qkv, int row_stride, const 
     const int head = r / units_per_head, u = r % units_per_head;
     const int i0 = u * 8;
     __nv_bfloat16* base = qkv + (size_t)t * row_stride + (size_t)head * D;
-    uint4 lo = *reinterpret_cast<const uint4*>(base + i0);
-    uint4 hi = *reinterpret_cast<const uint4*>(base + half + i0);
     const int seq = seq_ids[t], cp = cache_pos[t];
     const bool to_cache = head >= Hq && seq >= 0 && cp >= 0;
+    float x[8], y[8];
+    uint4 lo, hi;
+    if (slabs) {
+      const float* src = slabs + (size_t)t * (heads * D) + (size_t)head * D + i0;
+      slab_sum8(src, slab_stride, splits, x);
+      slab_sum8(src + half, slab_stride, splits, y);
+      if (bias) {
+        const uint4 blo = *reinterpret_cast<const uint4*>(bias + head * D + i0);
+        const uint4 bhi = *reinterpret_cast<const uint4*>(bias + head * D + half + i0);
+        const __nv_bfloat16 *a = reinterpret_cast<const __nv_bfloat16*>(&blo), *b = reinterpret_cast<const __nv_bfloat16*>(&bhi);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          x[k] += __bfloat162float(a[k]);
+          y[k] += __bfloat162float(b[k]);
+        }
+      }
+    } else {
+      lo = *reinterpret_cast<const uint4*>(base + i0);
+      hi = *reinterpret_cast<const uint4*>(base + half + i0);
+      const __nv_bfloat16 *a = reinterpret_cast<const __nv_bfloat16*>(&lo), *b = reinterpret_cast<const __nv_bfloat16*>(&hi);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x[k] = __bfloat162float(a[k]);
+        y[k] = __bfloat162float(b[k]);
+      }
+    }
     if (head < Hq + Hkv) {
-      __nv_bfloat16* a = reinterpret_cast<__nv_bfloat16*>(&lo);
-      __nv_bfloat16* b = reinterpret_cast<__nv_bfloat16*>(&hi);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const int i = i0 + k;
@@ -96,10 +119,14 @@ __global__ void rope_kv_append_kernel(__nv_bfloat16* qkv, int row_stride, const 
         if (pos_rows == 3) prow = (i < sec0) ? 0 : (i < sec1 ? 1 : 2);
         const int p = rope_pos[(size_t)prow * T + t];
         const float c = cos_tab[(size_t)p * half + i], s = sin_tab[(size_t)p * half + i];
-        const float x = __bfloat162float(a[k]), y = __bfloat162float(b[k]);
-        a[k] = __float2bfloat16(x * c - y * s);
-        b[k] = __float2bfloat16(y * c + x * s);
+        const float xr = x[k] * c - y[k] * s;
+        y[k] = y[k] * c + x[k] * s;
+        x[k] = xr;
       }
+    }
+    if (slabs || head < Hq + Hkv) {
+      lo = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+      hi = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]), pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
       *reinterpret_cast<uint4*>(base + i0) = lo;
       *reinterpret_cast<uint4*>(base + half + i0) = hi;
     }
@@ -399,18 +426,21 @@ extern "C" int sb_kv_append(const void* qkv, int row_stride, const int* seq_ids,
   return (int)cudaGetLastError();
 }
 
-extern "C" int sb_rope_kv_append(void* qkv, int row_stride, const int* rope_pos, int pos_rows, int sec0, int sec1,
+// slabs: null (qkv holds the projection) or the projection's fp32 partial sums [T, (Hq + 2 Hkv) * D], slab_stride floats
+// apart, to which `bias` (may be null) is added; the rows of qkv are then written whole
+extern "C" int sb_rope_kv_append(void* qkv, int row_stride, const float* slabs, long long slab_stride, int splits,
+                                 const void* bias, const int* rope_pos, int pos_rows, int sec0, int sec1,
                                  const float* cos_tab, const float* sin_tab, const int* seq_ids, const int* cache_pos,
                                  const int* block_table, int max_blocks, void* cache, int T, int Hq, int Hkv, int D,
                                  cudaStream_t stream) {
   if (T == 0) return 0;
-  if (D % 16) return -3;
+  if (D % 16 || (slabs && (splits < 1 || slab_stride % 4))) return -3;
   const long long total = (long long)T * (Hq + 2 * Hkv) * (D / 16);
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)num_sms() * 8;
   if (blocks > cap) blocks = cap;
-  return launch_chained(rope_kv_append_kernel, (unsigned)blocks, 256, 0, stream, (__nv_bfloat16*)qkv, row_stride, rope_pos,
-                        pos_rows, sec0, sec1, cos_tab, sin_tab, seq_ids, cache_pos, block_table, max_blocks,
+  return launch_chained(rope_kv_append_kernel, (unsigned)blocks, 256, 0, stream, (__nv_bfloat16*)qkv, row_stride, slabs,
+                        slab_stride, splits, (const __nv_bfloat16*)bias, rope_pos, pos_rows, sec0, sec1, cos_tab, sin_tab, seq_ids, cache_pos, block_table, max_blocks,
                         (__nv_bfloat16*)cache, T, Hq, Hkv, D);
 }
 

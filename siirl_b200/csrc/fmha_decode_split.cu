@@ -5,8 +5,8 @@
 // 32 KB stage in flight per CTA) and by the tail wave of a grid that is not a multiple of the resident slots.  Here:
 //   * one CTA per SM walks a list of work items (chunk, sequence, kv head); a sequence is cut into chunks of
 //     kChunkTiles cache blocks, so items are of similar size whatever the batch and the context lengths;
-//   * four working warps: warp 0 soft-max, warp 1 TMA producer, warp 2 MMA issuer, warp 4 output (warp 3 only makes
-//     warp 4 exist: rows 0..31 of TMEM belong to the warps whose index is a multiple of four).  The producer keeps a
+//   * four working warps: warp 0 soft-max, warp 1 TMA producer, warp 2 MMA issuer, warp 4 output (rows 0..31 of
+//     TMEM belong to the warps whose index is a multiple of four; warp 3 clears the rows of idle slots when no merge follows).  The producer keeps a
 //     ring of K/V stages full across item boundaries (128 KB in flight per SM at d = 128) and fetches the NEXT item's
 //     query rows while the current item runs; S is double-buffered in TMEM so the scores of tile t+1 are computed while
 //     tile t is in the soft-max, P is double-buffered in shared memory, and the output accumulator is double-buffered
@@ -592,6 +592,15 @@ fmha_decode_split_kernel(const __grid_constant__ CUtensorMap map_cache, const __
       }
       ++item_no;
     }
+  } else if (warp == 3) {
+    // ------------------------------ zero rows of idle slots, where no merge follows ------------------------------
+    if (MODE == 0 && p.max_chunks == 1) {
+      for (int b = blockIdx.x; b < p.B; b += gridDim.x) {
+        if (p.seq_lens[b] > 0) continue;
+        uint4* row = reinterpret_cast<uint4*>(p.out + (size_t)b * (p.Hq * D));
+        for (int i = lane; i < p.Hq * D / 8; i += 32) row[i] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
   } else if (warp == 4) {
     // ------------------------------ output (warp 4: TMEM lanes 0..31) ------------------------------
     uint32_t item_no = 0;
@@ -666,41 +675,45 @@ fmha_decode_split_kernel(const __grid_constant__ CUtensorMap map_cache, const __
   }
 }
 
-// merges the chunk partials of sequences longer than one chunk; zero rows for empty slots
+// merges the chunk partials of sequences longer than one chunk; zero rows for empty slots.  Four neighbouring columns per
+// thread: one block per head cost 5 us for 256 sequences of 28 heads, most of it blocks that had nothing to do.
 template <int D, bool WIN>
-__global__ void fmha_decode_merge_kernel(SplitParams p) {
+__global__ void __launch_bounds__(256) fmha_decode_merge_kernel(SplitParams p) {
   chain_sync();
-  const int b = blockIdx.x, h = blockIdx.y;
+  const int b = blockIdx.x;
   const int ctx = p.seq_lens[b];
   int n_tiles = (ctx + kSBlk - 1) / kSBlk;
   if constexpr (WIN) {
     int sinks, w0;
     visible_tiles(ctx, p.window, p.keep_first, p.pool, sinks, w0, n_tiles);
   }
+  if (ctx > 0 && n_tiles <= kChunkTiles) return;   // written by the attention kernel
+  const int at = (blockIdx.y * 256 + threadIdx.x) * 4, h = at / D, d = at % D;
   const int dv = WIN ? p.dv : D;
-  __nv_bfloat16* orow = p.out + (WIN ? (size_t)b * p.out_stride : (size_t)b * (p.Hq * D)) + (size_t)h * dv;
-  const int d = threadIdx.x;   // blockDim.x == D
-  if (WIN && d >= dv) return;
+  if (h >= p.Hq || d >= dv) return;
+  uint2* dst = reinterpret_cast<uint2*>(p.out + (WIN ? (size_t)b * p.out_stride : (size_t)b * (p.Hq * D)) + (size_t)h * dv + d);
   if (ctx <= 0) {
-    orow[d] = __float2bfloat16(0.f);
+    *dst = make_uint2(0u, 0u);
     return;
   }
-  if (n_tiles <= kChunkTiles) return;   // written by the attention kernel
   const int nc = (n_tiles + kChunkTiles - 1) / kChunkTiles;
   const float* lse = p.ws_lse + ((size_t)b * p.Hq + h) * p.max_chunks;
-  const float* wo = p.ws_o + ((size_t)b * p.Hq + h) * p.max_chunks * D;
+  const float* wo = p.ws_o + ((size_t)b * p.Hq + h) * p.max_chunks * D + d;
   float m = -INFINITY;
   for (int c = 0; c < nc; ++c) m = fmaxf(m, lse[c]);
-  float acc = 0.f, wsum = 0.f;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, wsum = 0.f;
   for (int c = 0; c < nc; ++c) {
     const float w = exp2f(lse[c] - m);
+    const float4 o = *reinterpret_cast<const float4*>(wo + (size_t)c * D);
     wsum += w;
-    acc += w * wo[(size_t)c * D + d];
+    acc[0] += w * o.x; acc[1] += w * o.y; acc[2] += w * o.z; acc[3] += w * o.w;
   }
   if (WIN) wsum += sink_term(p, h, m);
   float f = WIN ? p.out_scale : 1.f;
   if (WIN && p.head_gate) f *= p.head_gate[(size_t)b * p.Hq + h];
-  orow[d] = __float2bfloat16(wsum > 0.f ? acc / wsum * f : 0.f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i] = wsum > 0.f ? acc[i] / wsum * f : 0.f;
+  *dst = make_uint2(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]));
 }
 
 template <int D, int MODE>
@@ -717,8 +730,8 @@ static int launch_decode_split(const CUtensorMap& mc, const CUtensorMap& mv, con
   const int items = p.max_chunks * p.B * p.Hkv;
   const int grid = items < num_sms() ? items : num_sms();
   const int rc = launch_chained(kernel, grid, 160, L::kTotal, stream, mc, mv, mq, p);
-  if (rc) return rc;
-  return launch_chained(fmha_decode_merge_kernel<D, (MODE > 0)>, dim3(p.B, p.Hq), D, 0, stream, p);
+  if (rc || (MODE == 0 && p.max_chunks == 1)) return rc;
+  return launch_chained(fmha_decode_merge_kernel<D, (MODE > 0)>, dim3(p.B, (p.Hq * D + 1023) / 1024), 256, 0, stream, p);
 }
 
 }  // namespace sb

@@ -63,6 +63,9 @@ int sb_splitk_reduce(const float* slabs, long long slab_stride, int splits, cons
 // ---- elementwise.cu ----
 int sb_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* h_out, float* rstd,
                    int T, int H, float eps, cudaStream_t stream);
+int sb_rmsnorm_slabs_fwd(const float* slabs, long long slab_stride, int splits, const void* residual, const void* w, void* y,
+                         void* h_out, int T, int H, float eps, cudaStream_t stream);
+int sb_swiglu_slabs_fwd(const float* slabs, long long slab_stride, int splits, void* out, int T, int I, cudaStream_t stream);
 int sb_rmsnorm_bwd_blocks(int T);
 int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres, void* dx,
                    float* dw_partial, float* dw, int dw_accumulate, int T, int H, cudaStream_t stream);
@@ -127,7 +130,8 @@ extern "C" {
 // ---- fmha_decode.cu ----
 int sb_kv_append(const void* qkv, int row_stride, const int* seq_ids, const int* positions, const int* block_table,
                  int max_blocks, void* cache, int T, int Hq, int Hkv, int D, cudaStream_t stream);
-int sb_rope_kv_append(void* qkv, int row_stride, const int* rope_pos, int pos_rows, int sec0, int sec1,
+int sb_rope_kv_append(void* qkv, int row_stride, const float* slabs, long long slab_stride, int splits, const void* bias,
+                      const int* rope_pos, int pos_rows, int sec0, int sec1,
                       const float* cos_tab, const float* sin_tab, const int* seq_ids, const int* cache_pos,
                       const int* block_table, int max_blocks, void* cache, int T, int Hq, int Hkv, int D,
                       cudaStream_t stream);

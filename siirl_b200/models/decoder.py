@@ -243,6 +243,28 @@ class DecoderLayer(nn.Module):
             return leave_parallel_block(y, tp)
         return self._linear(ops.swiglu(self._linear(x, "gate_up_proj")), "down_proj")
 
+    # ---- few rows (decode): partial sums of split projections go straight to the kernel that consumes them ----
+    def project_cached(self, x: torch.Tensor, name: str) -> Optional[torch.Tensor]:
+        """fp32 partial sums ``[S, T, width]`` of a plain projection without its bias; ``None`` where it is not split."""
+        if hasattr(self, f"{name}_lora_A") and self.lora_enabled or getattr(self, "tp", None) is not None:
+            return None
+        return ops.linear_slabs(x, getattr(self, f"{name}_weight"))
+
+    def norm_cached(self, delta: Optional[torch.Tensor], h: torch.Tensor, weight: torch.Tensor):
+        """Norm of ``h + delta`` and the sum itself; ``delta`` may be partial sums or missing."""
+        eps = self.cfg.rms_norm_eps
+        if delta is None:
+            return ops.rmsnorm(h, weight, eps)
+        return ops.rmsnorm_slabs(delta, weight, eps, h) if delta.dim() == 3 else ops.rmsnorm(delta, weight, eps, residual=h)
+
+    def mlp_cached(self, x: torch.Tensor) -> torch.Tensor:
+        if self.is_moe or self.cfg.lora_rank > 0 or getattr(self, "tp", None) is not None:
+            return self.mlp(x)
+        gate_up = self.project_cached(x, "gate_up_proj")
+        a = ops.swiglu_slabs(gate_up) if gate_up is not None else ops.swiglu(self._linear(x, "gate_up_proj"))
+        y = self.project_cached(a, "down_proj")
+        return y if y is not None else self._linear(a, "down_proj")
+
     def forward(self, h: torch.Tensor, delta: Optional[torch.Tensor], positions, info: SeqInfo, rope, causal=True):
         """``h`` is the residual stream, ``delta`` the previous sub-layer output not yet added to it."""
         cfg = self.cfg
@@ -574,10 +596,12 @@ class DecoderLM(nn.Module):
             rp = rp[0]
         rp32 = rp.to(torch.int32).contiguous()
         for li, layer in enumerate(self.layers):
-            x, h = ops.rmsnorm(delta if delta is not None else h, layer.input_layernorm, cfg.rms_norm_eps,
-                               residual=h if delta is not None else None)
-            qkv = kvc.rope_kv_append(layer.qkv_pre_rope(x), rp32, rope[0], rope[1], cfg.mrope_section, seq_ids, pos32,
-                                     block_table, cache[li], cfg.num_heads, cfg.num_kv_heads, cfg.head_dim)
+            x, h = layer.norm_cached(delta, h, layer.input_layernorm)
+            qkv = layer.project_cached(x, "qkv_proj") if not cfg.qk_norm and cfg.head_dim % 16 == 0 else None
+            bias = layer.qkv_proj_bias if qkv is not None else None
+            qkv = kvc.rope_kv_append(qkv if qkv is not None else layer.qkv_pre_rope(x), rp32, rope[0], rope[1],
+                                     cfg.mrope_section, seq_ids, pos32, block_table, cache[li], cfg.num_heads,
+                                     cfg.num_kv_heads, cfg.head_dim, bias)
             if prefill_info is not None and prefix_lens is not None and any(int(p) > 0 for p in prefix_lens):
                 # chunked prefill / prefix-cache hit: the chunk attends to the tokens already in the cache as well
                 a = kvc.prefill_attention_with_prefix(qkv, prefill_info.seqlens, prefix_lens, prefill_slots, cache[li],
@@ -587,11 +611,11 @@ class DecoderLM(nn.Module):
             else:
                 a = kvc.decode_attention(qkv, cache[li], seq_lens, block_table, cfg.num_heads, cfg.num_kv_heads,
                                          cfg.head_dim)
-            attn_out = layer._linear(a, "o_proj")
-            x, h = ops.rmsnorm(attn_out, layer.post_attention_layernorm, cfg.rms_norm_eps, residual=h)
-            delta = layer.mlp(x)
-        out, _ = ops.rmsnorm(delta, self.norm, cfg.rms_norm_eps, residual=h)
-        return out
+            attn_out = layer.project_cached(a, "o_proj")
+            x, h = layer.norm_cached(attn_out if attn_out is not None else layer._linear(a, "o_proj"), h,
+                                     layer.post_attention_layernorm)
+            delta = layer.mlp_cached(x)
+        return self.layers[-1].norm_cached(delta, h, self.norm)[0]
 
     def named_flat_order(self) -> List[Tuple[str, nn.Parameter]]:
         return list(self.named_parameters())

@@ -206,6 +206,24 @@ def linear_skinny(x2: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
     return out
 
 
+def _row_splits(M: int, N: int, K: int) -> int:
+    """How often :func:`linear` splits the contraction of ``M <= 512`` rows."""
+    if M > 128 and SWAP_OPERANDS_ABOVE_128_ROWS:
+        return _best_splits((N + 127) // 128 * ((M + 255) // 256), (K + 63) // 64)
+    return _skinny_splits(M, N, K)
+
+
+def linear_slabs(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
+    """Inference-only: the fp32 partial sums ``[S, M, N]`` of ``x @ W^T`` where :func:`linear` would split the contraction
+    of so few rows and add them up in a launch of its own; ``None`` where it would not.  For consumers that add them
+    themselves (:func:`rmsnorm_slabs`, :func:`swiglu_slabs` and :func:`~siirl_b200.ops.kv_cache.rope_kv_append`)."""
+    M, K = x.shape
+    N = weight.shape[0]
+    if not x.is_cuda or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or M > 512 or K % 8 or N % 8:
+        return None
+    return linear_partial(x, weight) if _row_splits(M, N, K) > 1 else None
+
+
 def linear_partial(x: torch.Tensor, weight: torch.Tensor, f32: bool = False, max_splits: int = 0) -> torch.Tensor:
     """Inference-only ``x @ W^T`` as partial sums ``[S, M, N]`` for a consumer that adds them itself: few rows give the
     fp32 slabs of a split contraction, many rows one bf16 product (fp32 when ``f32``).  ``max_splits``: a product of few
@@ -221,7 +239,7 @@ def linear_partial(x: torch.Tensor, weight: torch.Tensor, f32: bool = False, max
         return gemm(x, weight, epi=EPI_F32 if f32 else EPI_BF16)[None]
     nkb = (K + 63) // 64
     swap = M > 128 and SWAP_OPERANDS_ABOVE_128_ROWS
-    splits = _best_splits((N + 127) // 128 * ((M + 255) // 256), nkb) if swap else _skinny_splits(M, N, K)
+    splits = _row_splits(M, N, K)
     if max_splits:
         splits = max(splits, min(max_splits, nkb // 2))
     if splits <= 1 and not f32:
@@ -312,6 +330,18 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: 
     return y.reshape(shp), (h.reshape(shp) if residual is not None else x)
 
 
+def rmsnorm_slabs(slabs: torch.Tensor, weight: torch.Tensor, eps: float, residual: torch.Tensor):
+    """Inference-only :func:`rmsnorm` of the partial sums ``[S, T, H]`` of :func:`linear_slabs` plus ``residual``."""
+    S, T, H = slabs.shape
+    assert slabs.is_contiguous() and slabs.dtype == torch.float32 and residual.shape == (T, H)
+    residual = residual.contiguous()
+    y, h = torch.empty_like(residual), torch.empty_like(residual)
+    _lib.check(_lib.get_lib().sb_rmsnorm_slabs_fwd(
+        _lib.ptr(slabs), ctypes.c_longlong(T * H), S, _lib.ptr(residual), _lib.ptr(weight), _lib.ptr(y), _lib.ptr(h), T, H,
+        ctypes.c_float(eps), _lib.stream()), "sb_rmsnorm_slabs_fwd")
+    return y, h
+
+
 # ---------------------------------------------------------------------------------------------
 # RoPE
 # ---------------------------------------------------------------------------------------------
@@ -393,6 +423,16 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     shp = gate_up.shape
     out = _SwiGLUFn.apply(gate_up.reshape(-1, shp[-1]).contiguous())
     return out.reshape(*shp[:-1], shp[-1] // 2)
+
+
+def swiglu_slabs(slabs: torch.Tensor) -> torch.Tensor:
+    """Inference-only :func:`swiglu` of the partial sums ``[S, T, 2I]`` of :func:`linear_slabs`."""
+    S, T, I2 = slabs.shape
+    assert slabs.is_contiguous() and slabs.dtype == torch.float32
+    out = torch.empty(T, I2 // 2, dtype=torch.bfloat16, device=slabs.device)
+    _lib.check(_lib.get_lib().sb_swiglu_slabs_fwd(_lib.ptr(slabs), ctypes.c_longlong(T * I2), S, _lib.ptr(out), T,
+                                                  I2 // 2, _lib.stream()), "sb_swiglu_slabs_fwd")
+    return out
 
 
 # ---------------------------------------------------------------------------------------------

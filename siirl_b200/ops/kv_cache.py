@@ -46,9 +46,16 @@ def kv_append(qkv: torch.Tensor, seq_ids: torch.Tensor, positions: torch.Tensor,
 
 def rope_kv_append(qkv: torch.Tensor, rope_positions: torch.Tensor, cos_tab: torch.Tensor, sin_tab: torch.Tensor,
                    mrope_section, seq_ids: torch.Tensor, cache_positions: torch.Tensor, block_table: torch.Tensor,
-                   cache_layer: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int) -> torch.Tensor:
+                   cache_layer: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int,
+                   bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Inference-only fusion of RoPE and cache append: rotates the q and k heads of ``qkv`` IN PLACE and writes the
-    rotated k and the v heads to the cache (one kernel on CUDA).  Returns ``qkv``."""
+    rotated k and the v heads to the cache (one kernel on CUDA).  Returns ``qkv``.  On CUDA ``qkv`` may be the partial sums
+    ``[S, T, width]`` of :func:`siirl_b200.ops.dense.linear_slabs`, which are added up with ``bias`` on the way."""
+    slabs = None
+    if qkv.dim() == 3:
+        slabs = qkv
+        assert slabs.is_cuda and slabs.is_contiguous() and slabs.dtype == torch.float32 and head_dim % 16 == 0
+        qkv = torch.empty(slabs.shape[1:], dtype=cache_layer.dtype, device=slabs.device)
     if qkv.is_cuda and head_dim % 16 == 0:
         L = _lib.get_lib()
         pos = rope_positions.to(torch.int32).contiguous()
@@ -56,7 +63,8 @@ def rope_kv_append(qkv: torch.Tensor, rope_positions: torch.Tensor, cos_tab: tor
         s0 = s1 = 0
         if rows == 3:
             s0, s1 = mrope_section[0], mrope_section[0] + mrope_section[1]
-        _lib.check(L.sb_rope_kv_append(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(pos), rows, s0, s1, _lib.ptr(cos_tab),
+        _lib.check(L.sb_rope_kv_append(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(slabs), ctypes.c_longlong(qkv.numel()),
+                                       slabs.shape[0] if slabs is not None else 0, _lib.ptr(bias), _lib.ptr(pos), rows, s0, s1, _lib.ptr(cos_tab),
                                        _lib.ptr(sin_tab), _lib.ptr(seq_ids), _lib.ptr(cache_positions),
                                        _lib.ptr(block_table), block_table.shape[1], _lib.ptr(cache_layer),
                                        qkv.shape[0], n_heads, n_kv_heads, head_dim, _lib.stream()),

@@ -206,3 +206,40 @@ def test_optimizer_state_offload_round_trip():
     sb.reload_state()
     assert torch.equal(sa.flat_param, sb.flat_param) and torch.equal(sa.exp_avg, sb.exp_avg)
     assert torch.equal(sa.exp_avg_sq, sb.exp_avg_sq)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 100, 129, 256, 300])
+@pytest.mark.parametrize("hidden,inter,hq,hkv,d", [(896, 2432, 14, 2, 64), (1024, 1536, 4, 4, 128)])
+def test_partial_sums_and_their_consumers(rows, hidden, inter, hq, hkv, d):
+    """Projections of few rows whose partial sums go to the norm, the gated activation, and rope with the cache append."""
+    from siirl_b200.ops import kv_cache as kvc
+    torch.manual_seed(0)
+    mk = lambda *s: (torch.randn(*s, device=DEV) / s[-1] ** 0.5).to(torch.bfloat16)  # noqa: E731
+    x = torch.randn(rows, hidden, device=DEV).to(torch.bfloat16)
+    h, w = torch.randn_like(x), (1 + 0.1 * torch.randn(hidden, device=DEV)).to(torch.bfloat16)
+    wo, wg, wq, bias = mk(hidden, hidden), mk(2 * inter, hidden), mk((hq + 2 * hkv) * d, hidden), mk((hq + 2 * hkv) * d)
+    so, sg, sq = (ops.linear_slabs(x, t) for t in (wo, wg, wq))
+    assert so is not None and sq is not None
+    y, hs = ops.rmsnorm_slabs(so, w, 1e-6, h)
+    want = x.double() @ wo.double().T + h.double()
+    # results rounded to bf16 once (2^-9 relative), the norm's input as well
+    assert ((hs.double() - want).norm() / want.norm()).item() < 3e-3
+    want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert ((y.double() - want).norm() / want.norm()).item() < 5e-3
+    if sg is not None:
+        g, u = (x.double() @ wg.double().T).chunk(2, -1)
+        want = torch.nn.functional.silu(g) * u
+        assert ((ops.swiglu_slabs(sg).double() - want).norm() / want.norm()).item() < 3e-3
+    cos, sin = ops.rope_tables(d, 64, 10000.0, device=DEV)
+    pos = (torch.arange(rows, device=DEV) % 64).to(torch.int32)
+    seq = torch.arange(rows, device=DEV, dtype=torch.int32)
+    seq[rows // 2] = -1
+    table = torch.arange(rows, device=DEV, dtype=torch.int32)[:, None].contiguous()
+    cache = [torch.zeros(rows, 2, hkv, 64, d, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    a = kvc.rope_kv_append(sq, pos, cos, sin, None, seq, pos, table, cache[0], hq, hkv, d, bias)
+    b = kvc.rope_kv_append(ops.linear(x, wq, bias), pos, cos, sin, None, seq, pos, table, cache[1], hq, hkv, d)
+    # the sums enter unrounded here, rounded to bf16 there
+    assert ((a.double() - b.double()).norm() / b.double().norm()).item() < 4e-3
+    assert ((cache[0].double() - cache[1].double()).norm() / (cache[1].double().norm() + 1e-9)).item() < 4e-3
+    for p, q in zip(*cache):
+        assert torch.equal(p.abs().sum(-1) != 0, q.abs().sum(-1) != 0)

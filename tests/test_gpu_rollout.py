@@ -85,3 +85,30 @@ def test_lora_adapters_forward_backward_on_gpu():
     assert (ga - gc).abs().max().item() < 0.05 * max(1.0, gc.abs().max().item()) + 1e-3
     torch.cuda.synchronize()
     lib.check_status()
+
+
+@pytest.mark.parametrize("d,hq,hkv", [(64, 14, 2), (128, 6, 2)])
+@pytest.mark.parametrize("max_blocks,lens", [(2, [0, 1, 64, 65, 128, 0]), (17, [0, 1024, 1025, 1088, 63, 0]),
+                                             (40, [0, 2560, 1, 1100, 0, 2049])])
+def test_decode_attention_of_idle_slots_and_chunks(d, hq, hkv, max_blocks, lens):
+    """One chunk (no merge pass), several, and slots without a sequence, whose rows are zero."""
+    from siirl_b200.ops import kv_cache as kvc, lib
+    torch.manual_seed(0)
+    B = len(lens)
+    cache = torch.randn(B * max_blocks, 2, hkv, 64, d, device="cuda").to(torch.bfloat16)
+    table = torch.randperm(B * max_blocks, device="cuda").to(torch.int32).reshape(B, max_blocks)
+    q = torch.randn(B, (hq + 2 * hkv) * d, device="cuda").to(torch.bfloat16)
+    out = torch.full((B, hq * d), 7.0, device="cuda", dtype=torch.bfloat16)
+    n = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    kvc.decode_attention(q, cache, n, table, hq, hkv, d, out=out)
+    lib.check_status()
+    for b, m in enumerate(lens):
+        if m == 0:
+            assert not out[b].any()
+            continue
+        kv = cache[table[b].long()].double().permute(1, 2, 0, 3, 4).reshape(2, hkv, -1, d)[:, :, :m]
+        k, v = (x.repeat_interleave(hq // hkv, 0) for x in kv)
+        s = torch.einsum("hd,hnd->hn", q[b, :hq * d].double().reshape(hq, d), k) / d ** 0.5
+        want = torch.einsum("hn,hnd->hd", torch.softmax(s, -1), v).reshape(-1)
+        # weights and result are rounded to bf16 (2^-9 each)
+        assert ((out[b].double() - want).norm() / want.norm()).item() < 1e-2

@@ -88,10 +88,9 @@ int sb_gae_scan(const float* rewards, const float* values, const float* mask, fl
 int sb_grpo_group_adv(const float* rewards, const float* mask, const int* gid, float* scores_ws, float* group_ws,
                       float* adv, int B, int R, int G, float eps, int norm_by_std, cudaStream_t stream);
 int sb_ppo_token_loss(const float* logp, const float* old_logp, const float* adv, const float* mask,
-                      const float* ref_logp, const float* entropy, const float* w_row, const float* seq_logratio,
-                      float* dlogp, float* dentropy, float* stats, int B, int R, int mode, float clip_lo,
-                      float clip_hi, float clip_c, int use_kl, float kl_coef, float entropy_coef,
-                      float loss_scale, cudaStream_t stream);
+                      const float* ref_logp, const float* entropy, float* rows_ws, float* dlogp, float* dentropy,
+                      float* stats, float* loss, int B, int R, int mode, int agg, float clip_lo, float clip_hi,
+                      float clip_c, int use_kl, float kl_coef, float entropy_coef, cudaStream_t stream);
 }
 
 extern "C" {

@@ -64,19 +64,7 @@ _KL_KIND = {None: 0, "low_var_kl": 1, "k3": 1, "kl": 2, "k1": 2, "abs": 3, "mse"
 _MODE = {"vanilla": 0, "gspo": 1, "cpgd": 2}
 
 
-def agg_row_weights(mask: torch.Tensor, loss_agg_mode: str) -> torch.Tensor:
-    """Per-row weight w_b such that the aggregated loss equals sum_bt w_b * m_bt * l_bt."""
-    B, R = mask.shape
-    mf = mask.float()
-    if loss_agg_mode == "token-mean":
-        return torch.full((B,), 1.0, device=mask.device) / (mf.sum() + 1e-8)
-    if loss_agg_mode == "seq-mean-token-sum":
-        return torch.full((B,), 1.0 / B, device=mask.device)
-    if loss_agg_mode == "seq-mean-token-mean":
-        return 1.0 / ((mf.sum(-1) + 1e-8) * B)
-    if loss_agg_mode == "seq-mean-token-sum-norm":
-        return torch.full((B,), 1.0 / R, device=mask.device)
-    raise ValueError(f"Invalid loss_agg_mode: {loss_agg_mode}")
+_AGG = {"token-mean": 0, "seq-mean-token-sum": 1, "seq-mean-token-mean": 2, "seq-mean-token-sum-norm": 3}
 
 
 class _PpoLossFn(torch.autograd.Function):
@@ -88,23 +76,25 @@ class _PpoLossFn(torch.autograd.Function):
         lp = logp.float().contiguous()
         mf = mask.float().contiguous()
         agg = "seq-mean-token-mean" if mode == "gspo" else loss_agg_mode
-        w = agg_row_weights(mf, agg).contiguous()
-        seq_lr = None
-        if mode == "gspo":
-            seq_lr = (((lp - old_logp.float()) * mf).sum(-1) / mf.sum(-1).clamp(min=1)).contiguous()
+        if agg not in _AGG:
+            raise ValueError(f"Invalid loss_agg_mode: {agg}")
         dlogp = torch.empty_like(lp)
         ent = entropy.float().contiguous() if entropy is not None else None
         dent = torch.empty_like(lp) if ent is not None else None
-        stats = torch.empty(8, dtype=torch.float32, device=lp.device)
+        rows = torch.empty(2 * B, dtype=torch.float32, device=lp.device)
+        stats = torch.empty(16, dtype=torch.float32, device=lp.device)
+        total = torch.empty((), dtype=torch.float32, device=lp.device)
+        if lp.numel() == 0:
+            stats.zero_()
+            total.zero_()
         _lib.check(L.sb_ppo_token_loss(
             _lib.ptr(lp), _lib.ptr(old_logp.float().contiguous()), _lib.ptr(adv.float().contiguous()),
             _lib.ptr(mf), _lib.ptr(ref_logp.float().contiguous() if ref_logp is not None else None),
-            _lib.ptr(ent), _lib.ptr(w), _lib.ptr(seq_lr), _lib.ptr(dlogp), _lib.ptr(dent), _lib.ptr(stats), B, R,
-            _MODE[mode], _f(clip_lo), _f(clip_hi), _f(clip_c), _KL_KIND[kl_kind if ref_logp is not None else None],
-            _f(kl_coef), _f(entropy_coef), _f(1.0), _lib.stream()), "sb_ppo_token_loss")
+            _lib.ptr(ent), _lib.ptr(rows), _lib.ptr(dlogp), _lib.ptr(dent), _lib.ptr(stats), _lib.ptr(total), B, R,
+            _MODE[mode], _AGG[agg], _f(clip_lo), _f(clip_hi), _f(clip_c),
+            _KL_KIND[kl_kind if ref_logp is not None else None], _f(kl_coef), _f(entropy_coef), _lib.stream()),
+            "sb_ppo_token_loss")
         ctx.save_for_backward(dlogp, dent)
-        pg_loss, kl_loss, ent_loss = stats[0], stats[4], stats[5]
-        total = pg_loss + kl_coef * kl_loss - entropy_coef * ent_loss
         ctx.mark_non_differentiable(stats)
         return total, stats
 
@@ -126,7 +116,6 @@ def ppo_token_loss(logp, old_logp, adv, mask, *, entropy=None, ref_logp=None, mo
     assert logp.is_cuda
     total, stats = _PpoLossFn.apply(logp, entropy, old_logp, adv, mask, ref_logp, mode, loss_agg_mode, clip_lo,
                                     clip_hi, clip_c, kl_kind, kl_coef, entropy_coef)
-    msum = stats[6].clamp(min=1e-8)
-    metrics = {"pg_loss": stats[0], "pg_clipfrac": stats[1] / msum, "ppo_kl": stats[2] / msum,
-               "pg_clipfrac_lower": stats[3] / msum, "kl_loss": stats[4], "entropy_loss": stats[5]}
+    metrics = {"pg_loss": stats[0], "pg_clipfrac": stats[8], "ppo_kl": stats[9], "pg_clipfrac_lower": stats[10],
+               "kl_loss": stats[4], "entropy_loss": stats[5]}
     return total, metrics

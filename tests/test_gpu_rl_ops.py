@@ -42,6 +42,46 @@ def test_grpo_group_adv_matches_formula():
     torch.testing.assert_close(got.cpu(), want, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("B,R,G", [(1, 1, 1), (2048, 5, 300), (2049, 5, 300), (9, 2100, 2)])
+def test_grpo_group_adv_sizes(B, R, G):
+    """Both forms of the group statistics (rows up to and above the scan's limit) and more columns than one sweep."""
+    g = torch.Generator().manual_seed(3)
+    rewards, m = torch.randn(B, R, generator=g), (torch.rand(B, R, generator=g) < 0.7).float()
+    gid = torch.randint(0, G, (B,), generator=g)
+    s = rewards.double().sum(-1)
+    want = torch.zeros(B, dtype=torch.float64)
+    for k in range(G):
+        at = gid == k
+        one = int(at.sum()) == 1
+        want[at] = (s[at] - (0.0 if one else s[at].mean())) / ((1.0 if one else s[at].std()) + 1e-6)
+    got = rl.grpo_group_advantage(rewards.to(DEV), m.to(DEV), gid.to(DEV), G)
+    # groups of two close scores divide small differences of 32-bit sums
+    torch.testing.assert_close(got.cpu().double(), want[:, None] * m, rtol=1e-3, atol=1e-4)
+
+
+@pytest.mark.parametrize("B,R", [(1, 1), (3, 257), (1200, 33), (2, 5000)])
+def test_ppo_loss_sizes(B, R):
+    """One token, rows and columns beyond one sweep of the grid; every token against 64 bits."""
+    torch.manual_seed(4)
+    m = (torch.rand(B, R, device=DEV) < 0.8).float()
+    m[:, 0] = 1
+    old, adv = -torch.rand(B, R, device=DEV) * 3, torch.randn(B, R, device=DEV)
+    logp = (old + 0.3 * torch.randn(B, R, device=DEV)).requires_grad_()
+    loss, met = rl.ppo_token_loss(logp, old, adv, m, mode="gspo")
+    loss.backward()
+    lp = logp.detach().double().requires_grad_()
+    mean = (((lp - old) * m).sum(-1) / m.sum(-1)).detach()
+    ratio = torch.exp(mean[:, None] + lp - lp.detach())
+    pg = torch.maximum(-adv * ratio, -adv * ratio.clamp(0.8, 1.2))
+    want = ((pg * m).sum(-1) / m.sum(-1)).mean()
+    want.backward()
+    torch.testing.assert_close(loss.double(), want, rtol=1e-4, atol=1e-5)
+    # ratios at the clip's edge apart, gradients agree to 32-bit rounding
+    near = ((ratio.detach() - 0.8).abs() < 1e-5) | ((ratio.detach() - 1.2).abs() < 1e-5)
+    assert ((logp.grad.double() - lp.grad).abs() * ~near).max() <= 1e-4 * lp.grad.abs().max() + 1e-9
+    torch.testing.assert_close(met["pg_loss"].double(), want.detach(), rtol=1e-4, atol=1e-5)
+
+
 @pytest.mark.parametrize("mode", ["vanilla", "gspo", "cpgd"])
 @pytest.mark.parametrize("agg", ["token-mean", "seq-mean-token-sum", "seq-mean-token-mean", "seq-mean-token-sum-norm"])
 def test_fused_ppo_loss_matches_torch(mode, agg):

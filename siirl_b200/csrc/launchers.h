@@ -71,6 +71,8 @@ int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rs
                    float* dw_partial, float* dw, int dw_accumulate, int T, int H, cudaStream_t stream);
 int sb_rope(void* qkv, const int* pos, const float* cos_tab, const float* sin_tab, int T, int row_stride,
             int n_heads_rot, int D, int pos_rows, int sec0, int sec1, float sign, cudaStream_t stream);
+int sb_rope_rows(const void* in, void* out, const int* pos, const float* cos_tab, const float* sin_tab, int T, int row_stride,
+                 int n_heads_rot, int D, int pos_rows, int sec0, int sec1, float sign, cudaStream_t stream);
 int sb_swiglu_fwd(const void* gu, void* out, int T, int I, cudaStream_t stream);
 int sb_swiglu_bwd(const void* gu, const void* dout, void* dgu, int T, int I, cudaStream_t stream);
 int sb_embedding_fwd(const long long* ids, const void* table, void* out, int T, int H, int V,

@@ -349,7 +349,8 @@ rope_tables = ref.rope_tables
 
 
 def _rope_native(qkv: torch.Tensor, n_heads_rot: int, head_dim: int, positions: torch.Tensor, cos_tab, sin_tab,
-                 mrope_section, sign: float) -> None:
+                 mrope_section, sign: float) -> torch.Tensor:
+    """Rotated copy of contiguous rows."""
     L = _lib.get_lib()
     T = qkv.shape[0]
     pos = positions.to(torch.int32).contiguous()
@@ -357,26 +358,29 @@ def _rope_native(qkv: torch.Tensor, n_heads_rot: int, head_dim: int, positions: 
     s0 = s1 = 0
     if rows == 3:
         s0, s1 = mrope_section[0], mrope_section[0] + mrope_section[1]
-    rc = L.sb_rope(_lib.ptr(qkv), _lib.ptr(pos), _lib.ptr(cos_tab), _lib.ptr(sin_tab), T, qkv.stride(0),
-                   n_heads_rot, head_dim, rows, s0, s1, ctypes.c_float(sign), _lib.stream())
+    out = torch.empty_like(qkv)
+    args = (_lib.ptr(pos), _lib.ptr(cos_tab), _lib.ptr(sin_tab), T, qkv.stride(0), n_heads_rot, head_dim, rows, s0, s1,
+            ctypes.c_float(sign), _lib.stream())
+    rc = L.sb_rope_rows(_lib.ptr(qkv), _lib.ptr(out), *args)
+    if rc == -2:        # odd widths
+        out.copy_(qkv)
+        rc = L.sb_rope(_lib.ptr(out), *args)
     _lib.check(rc, "sb_rope")
+    return out
 
 
 class _RopeFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, n_heads_rot, head_dim, positions, cos_tab, sin_tab, mrope_section):
-        out = qkv.clone()
-        _rope_native(out, n_heads_rot, head_dim, positions, cos_tab, sin_tab, mrope_section, 1.0)
         ctx.save_for_backward(positions, cos_tab, sin_tab)
         ctx.meta = (n_heads_rot, head_dim, mrope_section)
-        return out
+        return _rope_native(qkv, n_heads_rot, head_dim, positions, cos_tab, sin_tab, mrope_section, 1.0)
 
     @staticmethod
     def backward(ctx, dout):
         positions, cos_tab, sin_tab = ctx.saved_tensors
         n_heads_rot, head_dim, mrope_section = ctx.meta
-        d = dout.clone()
-        _rope_native(d, n_heads_rot, head_dim, positions, cos_tab, sin_tab, mrope_section, -1.0)
+        d = _rope_native(dout.contiguous(), n_heads_rot, head_dim, positions, cos_tab, sin_tab, mrope_section, -1.0)
         return d, None, None, None, None, None, None
 
 

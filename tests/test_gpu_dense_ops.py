@@ -243,3 +243,38 @@ def test_partial_sums_and_their_consumers(rows, hidden, inter, hq, hkv, d):
     assert ((cache[0].double() - cache[1].double()).norm() / (cache[1].double().norm() + 1e-9)).item() < 4e-3
     for p, q in zip(*cache):
         assert torch.equal(p.abs().sum(-1) != 0, q.abs().sum(-1) != 0)
+
+
+@pytest.mark.parametrize("T,heads,rot,d,mrope", [(1, 18, 16, 64, None), (300, 36, 32, 128, None), (77, 6, 6, 16, None),
+                                                 (130, 8, 5, 128, [16, 24, 24]), (9, 5, 3, 24, None)])
+def test_rope_rows(T, heads, rot, d, mrope):
+    """Rotated and copied heads, three position rows, and a width that takes the copy and the scalar kernel."""
+    torch.manual_seed(0)
+    x = torch.randn(T, heads * d, device=DEV).to(torch.bfloat16).requires_grad_()
+    cos, sin = ops.rope_tables(d, 512, 10000.0, device=DEV)
+    pos = torch.randint(0, 512, (3, T) if mrope else (T,), device=DEV)
+    y = ops.rope(x, rot, d, pos, cos, sin, mrope)
+    g = torch.randn_like(y)
+    y.backward(g)
+    for src, got, inverse in ((x.detach(), y.detach(), False), (g, x.grad, True)):
+        want = ref.rope(src[:, :rot * d].double().reshape(T, rot, d), pos, cos.double(), sin.double(), mrope,
+                        inverse).reshape(T, rot * d)
+        # one rounding to bf16: 2^-9 of the larger operand
+        assert (got[:, :rot * d].double() - want).abs().max() <= 2 ** -8 * want.abs().max()
+        assert torch.equal(got[:, rot * d:], src[:, rot * d:])
+
+
+@pytest.mark.parametrize("T,I", [(1, 8), (2, 1024), (3, 1032), (301, 4864), (5000, 264)])
+def test_swiglu_rows(T, I):
+    torch.manual_seed(0)
+    gu = (2 * torch.randn(T, 2 * I, device=DEV)).to(torch.bfloat16).requires_grad_()
+    y = ops.swiglu(gu)
+    d = torch.randn_like(y)
+    y.backward(d)
+    x = gu.detach().double().requires_grad_()
+    a, b = x.chunk(2, -1)
+    want = torch.nn.functional.silu(a) * b
+    want.backward(d.double())
+    # one rounding to bf16 each (2^-9 relative)
+    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
+    assert ((gu.grad.double() - x.grad).abs() <= 2 ** -8 * x.grad.abs() + 1e-5).all()

@@ -1124,16 +1124,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias, in
     };
     BN = (N > 128 && waves_cost(256, 1.0) <= waves_cost(128, 0.75)) ? 256 : 128;
   }
-  CUtensorMap ma, mb;
   int r;
-  if (!a_mn) r = make_tensor_map_bf16_2d(&ma, A, K, M, lda, kBK, kBM);
-  else r = make_tensor_map_bf16_2d(&ma, A, M, K, lda, 64, kBK);
-  if (r) return r;
-  const bool by_m = grp && grp->tile_group;
-  const long long b_groups = by_m ? grp->num_groups : 1;
-  if (!b_mn) r = make_tensor_map_bf16_2d(&mb, B, K, by_m ? b_groups * grp->b_group_rows : N, ldb, kBK, BN);
-  else r = make_tensor_map_bf16_2d(&mb, B, N, by_m ? b_groups * grp->b_group_rows : K, ldb, 64, kBK);
-  if (r) return r;
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc;
@@ -1193,6 +1184,15 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias, in
     const int rc = dispatch_pair(pa, pb, p, a_mn, b_mn, epi, stream);
     if (rc != -2) return rc;
   }
+  CUtensorMap ma, mb;
+  if (!a_mn) r = make_tensor_map_bf16_2d(&ma, A, K, M, lda, kBK, kBM);
+  else r = make_tensor_map_bf16_2d(&ma, A, M, K, lda, 64, kBK);
+  if (r) return r;
+  const bool by_m = grp && grp->tile_group;
+  const long long b_groups = by_m ? grp->num_groups : 1;
+  if (!b_mn) r = make_tensor_map_bf16_2d(&mb, B, K, by_m ? b_groups * grp->b_group_rows : N, ldb, kBK, BN);
+  else r = make_tensor_map_bf16_2d(&mb, B, N, by_m ? b_groups * grp->b_group_rows : K, ldb, 64, kBK);
+  if (r) return r;
   if (BN == 256) return dispatch_gemm<256, 4>(ma, mb, p, a_mn, b_mn, epi, max_ctas, stream);
   return dispatch_gemm<128, 6>(ma, mb, p, a_mn, b_mn, epi, max_ctas, stream);
 }

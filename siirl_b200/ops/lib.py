@@ -144,7 +144,9 @@ def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Current stream of the current device.  Asked for at every launch: the stream object that
+    ``torch.cuda.current_stream()`` makes on the way took a quarter of a launch's host time."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def status_word(device: Optional[torch.device] = None) -> torch.Tensor:

@@ -108,19 +108,19 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* x, const float* slabs, long long slab_st
 // RMSNorm backward.  dx = rstd * (g - xhat * mean(g * xhat)),  g = dy * w,  xhat = h * rstd.
 // dx is optionally added to `dres` (gradient arriving through the residual branch).
 // Per-block partial dw rows go to dw_partial[gridDim.x, H]; a second kernel folds them into fp32 dw.
-template <int CH>
-__global__ void __launch_bounds__(kNormThreads)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
-                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                   float* __restrict__ dw_partial, int T, int H) {
+// THREADS 128: rows of at most 1024 columns, four blocks per SM (9600 x 896: 256 threads, two blocks, 38 us).
+template <int THREADS, int CH>
+__global__ void __launch_bounds__(THREADS)
+rmsnorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* h, const __nv_bfloat16* w, const float* rstd,
+                   const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw_partial, int T, int H) {
   __shared__ float red[32];
+  chain_sync();
   const int nvec = H / 8;
   float dwacc[CH][8];
   float wv[CH][8];
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
-    const int vi = threadIdx.x + c * kNormThreads;
+    const int vi = threadIdx.x + c * THREADS;
 #pragma unroll
     for (int i = 0; i < 8; ++i) dwacc[c][i] = 0.f;
     if (vi < nvec) bf16x8_to_float(reinterpret_cast<const uint4*>(w)[vi], wv[c]);
@@ -131,7 +131,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     float dot = 0.f;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      const int vi = threadIdx.x + c * kNormThreads;
+      const int vi = threadIdx.x + c * THREADS;
       if (vi < nvec) {
         float dyv[8], hv[8];
         bf16x8_to_float(reinterpret_cast<const uint4*>(dy + (size_t)row * H)[vi], dyv);
@@ -145,10 +145,10 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
         }
       }
     }
-    const float mean = block_sum<kNormThreads>(dot, red) / (float)H;
+    const float mean = block_sum<THREADS>(dot, red) / (float)H;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      const int vi = threadIdx.x + c * kNormThreads;
+      const int vi = threadIdx.x + c * THREADS;
       if (vi < nvec) {
         float o[8];
 #pragma unroll
@@ -165,7 +165,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
-    const int vi = threadIdx.x + c * kNormThreads;
+    const int vi = threadIdx.x + c * THREADS;
     if (vi < nvec) {
       float4* dst = reinterpret_cast<float4*>(dw_partial + (size_t)blockIdx.x * H + (size_t)vi * 8);
       dst[0] = make_float4(dwacc[c][0], dwacc[c][1], dwacc[c][2], dwacc[c][3]);
@@ -174,13 +174,58 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-__global__ void colsum_accumulate_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows,
-                                         int H, int accumulate) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= H) return;
+// out[col] (+)= sum of `rows` partial rows.  32 columns and 8 groups of rows per block: with one thread per column the chain
+// of 296 dependent additions took 11.5 us for 896 columns.
+__global__ void __launch_bounds__(256) colsum_accumulate_kernel(const float* partial, float* out, int rows, int H,
+                                                                int accumulate) {
+  chain_sync();
+  __shared__ float red[8][33];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += partial[(size_t)r * H + col];
-  out[col] = accumulate ? out[col] + s : s;
+  if (col < H) {
+#pragma unroll 4
+    for (int r = grp; r < rows; r += 8) s += partial[(size_t)r * H + col];
+  }
+  red[grp][lane] = s;
+  __syncthreads();
+  if (grp == 0 && col < H) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) s += red[i][lane];
+    out[col] = accumulate ? out[col] + s : s;
+  }
+}
+
+// partial[block, :] = column sums of this block's rows of a bf16 matrix [T, N] (bias gradients); eight columns per thread
+__global__ void __launch_bounds__(128) colsum_rows_kernel(const __nv_bfloat16* x, float* partial, int T, int N) {
+  chain_sync();
+  const int v = blockIdx.x * 128 + threadIdx.x;
+  if (v >= N / 8) return;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+  for (int t = blockIdx.y; t < T; t += gridDim.y) {
+    float f[8];
+    bf16x8_to_float(reinterpret_cast<const uint4*>(x + (size_t)t * N)[v], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] += f[i];
+  }
+  float4* dst = reinterpret_cast<float4*>(partial + (size_t)blockIdx.y * N + (size_t)v * 8);
+  dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+}
+
+// out += sum over `splits` slabs (weight gradients of split contractions)
+__global__ void __launch_bounds__(256) slab_accumulate_kernel(const float* slabs, long long slab_stride, int splits, float* out,
+                                                              long long n4) {
+  chain_sync();
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n4; i += gridDim.x * 256ll) {
+    float4 a = reinterpret_cast<const float4*>(out)[i];
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      const float4 b = reinterpret_cast<const float4*>(slabs + s * slab_stride)[i];
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    }
+    reinterpret_cast<float4*>(out)[i] = a;
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -451,9 +496,14 @@ extern "C" int sb_rmsnorm_slabs_fwd(const float* slabs, long long slab_stride, i
   return rmsnorm_fwd(nullptr, slabs, slab_stride, splits, residual, w, y, h_out, nullptr, T, H, eps, stream);
 }
 
-extern "C" int sb_rmsnorm_bwd_blocks(int T) {
-  const int cap = num_sms() * 2;
+// rows of dw_partial that sb_rmsnorm_bwd writes for T rows of H columns
+extern "C" int sb_rmsnorm_bwd_blocks(int T, int H) {
+  const int cap = num_sms() * (H <= 1024 ? 4 : 2);
   return T < cap ? (T > 0 ? T : 1) : cap;
+}
+
+static int colsum_accumulate(const float* partial, float* out, int rows, int H, int accumulate, cudaStream_t stream) {
+  return launch_chained(colsum_accumulate_kernel, (H + 31) / 32, 256, 0, stream, partial, out, rows, H, accumulate);
 }
 
 extern "C" int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres,
@@ -462,20 +512,43 @@ extern "C" int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
   if (H % 8 || H > kNormThreads * 8 * kNormMaxChunks) return -3;
   if (T == 0) return 0;
   const int ch = (H / 8 + kNormThreads - 1) / kNormThreads;
-  const int grid = sb_rmsnorm_bwd_blocks(T);
-#define SB_LAUNCH(CH)                                                                                       \
-  rmsnorm_bwd_kernel<CH><<<grid, kNormThreads, 0, stream>>>(                                                \
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd,                      \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, T, H)
-  switch (ch) {
-    case 1: SB_LAUNCH(1); break;
-    case 2: SB_LAUNCH(2); break;
-    case 3: SB_LAUNCH(3); break;
-    default: SB_LAUNCH(4); break;
-  }
+  const int grid = sb_rmsnorm_bwd_blocks(T, H);
+  int rc;
+#define SB_LAUNCH(THREADS, CH)                                                                              \
+  rc = launch_chained(rmsnorm_bwd_kernel<THREADS, CH>, grid, THREADS, 0, stream, (const __nv_bfloat16*)dy,  \
+                      (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,   \
+                      (__nv_bfloat16*)dx, dw_partial, T, H)
+  if (H <= 1024) SB_LAUNCH(128, 1);
+  else if (ch == 1) SB_LAUNCH(kNormThreads, 1);
+  else if (ch == 2) SB_LAUNCH(kNormThreads, 2);
+  else if (ch == 3) SB_LAUNCH(kNormThreads, 3);
+  else SB_LAUNCH(kNormThreads, 4);
 #undef SB_LAUNCH
-  colsum_accumulate_kernel<<<(H + 127) / 128, 128, 0, stream>>>(dw_partial, dw, grid, H, dw_accumulate);
-  return (int)cudaGetLastError();
+  return rc ? rc : colsum_accumulate(dw_partial, dw, grid, H, dw_accumulate, stream);
+}
+
+extern "C" int sb_colsum_blocks(int T) {
+  const int rows = (T + 31) / 32;
+  return rows < 128 ? (rows > 0 ? rows : 1) : 128;
+}
+
+// out[N] (+)= column sums of x [T, N] bf16; partial: fp32 [sb_colsum_blocks(T), N]
+extern "C" int sb_colsum_bf16(const void* x, float* partial, float* out, int T, int N, int accumulate, cudaStream_t stream) {
+  if (N % 8 || ((uintptr_t)x & 15)) return -3;
+  if (N == 0) return 0;
+  const int gy = sb_colsum_blocks(T);
+  const int rc = launch_chained(colsum_rows_kernel, dim3((N / 8 + 127) / 128, gy), 128, 0, stream, (const __nv_bfloat16*)x,
+                                partial, T, N);
+  return rc ? rc : colsum_accumulate(partial, out, gy, N, accumulate, stream);
+}
+
+// out[n] += sum of `splits` slabs of n floats, slab_stride apart
+extern "C" int sb_slab_accumulate(const float* slabs, long long slab_stride, int splits, float* out, long long n,
+                                  cudaStream_t stream) {
+  if (n % 4 || slab_stride % 4 || ((uintptr_t)out & 15)) return -3;
+  if (n == 0) return 0;
+  return launch_chained(slab_accumulate_kernel, grid_for(n / 4, 256, 16), 256, 0, stream, slabs, slab_stride, splits, out,
+                        n / 4);
 }
 
 extern "C" int sb_rope(void* qkv, const int* pos, const float* cos_tab, const float* sin_tab, int T,

@@ -66,7 +66,10 @@ int sb_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, 
 int sb_rmsnorm_slabs_fwd(const float* slabs, long long slab_stride, int splits, const void* residual, const void* w, void* y,
                          void* h_out, int T, int H, float eps, cudaStream_t stream);
 int sb_swiglu_slabs_fwd(const float* slabs, long long slab_stride, int splits, void* out, int T, int I, cudaStream_t stream);
-int sb_rmsnorm_bwd_blocks(int T);
+int sb_rmsnorm_bwd_blocks(int T, int H);
+int sb_colsum_blocks(int T);
+int sb_colsum_bf16(const void* x, float* partial, float* out, int T, int N, int accumulate, cudaStream_t stream);
+int sb_slab_accumulate(const float* slabs, long long slab_stride, int splits, float* out, long long n, cudaStream_t stream);
 int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres, void* dx,
                    float* dw_partial, float* dw, int dw_accumulate, int T, int H, cudaStream_t stream);
 int sb_rope(void* qkv, const int* pos, const float* cos_tab, const float* sin_tab, int T, int row_stride,

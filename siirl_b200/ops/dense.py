@@ -20,6 +20,7 @@ from . import lib as _lib
 from . import reference as ref
 
 EPI_BF16, EPI_F32_ACC, EPI_F32 = 0, 1, 2
+_NUM_SMS = 148
 EPI_BF16_T, EPI_F32_T = 4, 5        # transposed stores of the "weights in the A operand" form (see linear_skinny)
 
 
@@ -72,6 +73,52 @@ def set_pair_kernel(enabled: bool) -> bool:
     return bool(_lib.get_lib().sb_gemm_set_pair_kernel(int(bool(enabled))))
 
 
+def _column_sums(x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """fp32 column sums of ``x [T, N]``, added to ``out`` when it is given."""
+    T, N = x.shape
+    if x.dtype != torch.bfloat16 or N % 8 or x.data_ptr() % 16 or (out is not None and not out.is_contiguous()):
+        s = x.float().sum(0)
+        return s if out is None else out.add_(s)
+    L = _lib.get_lib()
+    partial = torch.empty(L.sb_colsum_blocks(T), N, dtype=torch.float32, device=x.device)
+    acc = out is not None
+    out = out if acc else torch.empty(N, dtype=torch.float32, device=x.device)
+    _lib.check(L.sb_colsum_bf16(_lib.ptr(x), _lib.ptr(partial), _lib.ptr(out), T, N, int(acc), _lib.stream()),
+               "sb_colsum_bf16")
+    return out
+
+
+def _grad_splits(M: int, N: int, K: int) -> int:
+    """Contraction splits of a weight gradient ``[M, N]`` over ``K`` tokens.  A CTA pair takes about 0.4 us for a k-block of
+    its 256 x 256 tile and every split costs a pass over the slabs: matrices of few tiles leave most pairs idle
+    (1152 x 896 over 9600 tokens: 20 tiles for 74 pairs, 80 us), larger ones are left whole."""
+    tiles, nkb = -(-M // 256) * -(-N // 256), -(-K // 64)
+
+    def cost(s):
+        per = -(-nkb // s)
+        waves = -(-tiles * s // (_NUM_SMS // 2))
+        return waves * (0.4 * per + 3.0) + (4.0 + 2.4e-6 * s * M * N if s > 1 else 0.0)
+    best = min(range(1, 9), key=cost)
+    return best if best > 1 and nkb >= 4 * best and cost(best) < 0.8 * cost(1) else 1
+
+
+def _accumulate_weight_grad(dy: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> None:
+    """``out += dy^T x`` in fp32."""
+    K, M = dy.shape
+    N = x.shape[1]
+    splits = _grad_splits(M, N, K) if M > 128 and N >= 128 and out.is_contiguous() and out.data_ptr() % 16 == 0 else 1
+    if splits == 1:
+        gemm(dy, x, out=out, a_mn=True, b_mn=True, epi=EPI_F32_ACC)
+        return
+    nkb = (K + 63) // 64
+    per = (nkb + splits - 1) // splits
+    splits = (nkb + per - 1) // per
+    slabs = torch.empty(splits, M, N, dtype=torch.float32, device=dy.device)
+    gemm(dy, x, out=slabs[0], a_mn=True, b_mn=True, epi=EPI_F32, k_splits=splits, slab_stride=M * N)
+    _lib.check(_lib.get_lib().sb_slab_accumulate(_lib.ptr(slabs), ctypes.c_longlong(M * N), splits, _lib.ptr(out),
+                                                 ctypes.c_longlong(M * N), _lib.stream()), "sb_slab_accumulate")
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -99,21 +146,19 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             mg = getattr(ctx.weight_ref, "main_grad", None)
             if mg is not None:
-                gemm(dy2, x2, out=mg, a_mn=True, b_mn=True, epi=EPI_F32_ACC)
+                _accumulate_weight_grad(dy2, x2, mg)
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True, epi=EPI_F32).to(weight.dtype)
         db = None
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            bsum = dy2.float().sum(0)
             mgb = getattr(ctx.bias_ref, "main_grad", None)
             if mgb is not None:
-                mgb.add_(bsum)
+                _column_sums(dy2, mgb)
             else:
-                db = bsum.to(dy.dtype)
+                db = _column_sums(dy2).to(dy.dtype)
         return dx, dw, db
 
 
-_NUM_SMS = 148
 _ONE_WAVE = 100      # from this many tiles on, the partial sums of a split cost more than the SMs that stay idle without one
 SWAP_OPERANDS_ABOVE_128_ROWS = True     # benchmarks flip this to time both forms
 
@@ -306,7 +351,7 @@ class _RMSNormFn(torch.autograd.Function):
         T, H = h.shape
         dy = dy.contiguous()
         dx = torch.empty_like(h)
-        nblk = L.sb_rmsnorm_bwd_blocks(T)
+        nblk = L.sb_rmsnorm_bwd_blocks(T, H)
         partial = torch.empty(nblk, H, dtype=torch.float32, device=h.device)
         mg = getattr(ctx.weight_ref, "main_grad", None)
         dw_buf = mg if mg is not None else torch.empty(H, dtype=torch.float32, device=h.device)

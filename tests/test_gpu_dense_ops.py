@@ -278,3 +278,45 @@ def test_swiglu_rows(T, I):
     # one rounding to bf16 each (2^-9 relative)
     assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
     assert ((gu.grad.double() - x.grad).abs() <= 2 ** -8 * x.grad.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("M,N,K,splits", [(1152, 896, 9600, 3), (136, 128, 4104, 8), (896, 896, 1000, 1), (9728, 896, 4096, 1)])
+def test_weight_gradient_splits(M, N, K, splits):
+    """Contractions of few tiles are split over the tokens; the sums are added to what the gradient holds."""
+    got = dense._grad_splits(M, N, K)
+    assert (got > 1) == (splits > 1), got
+    torch.manual_seed(0)
+    dy, x = (torch.randn(K, n, device=DEV).to(torch.bfloat16) for n in (M, N))
+    out = torch.randn(M, N, device=DEV)
+    want = out.double() + dy.double().T @ x.double()
+    dense._accumulate_weight_grad(dy, x, out)
+    lib.check_status()
+    assert ((out.double() - want).norm() / want.norm()).item() < 1e-5      # 32-bit sums
+
+
+@pytest.mark.parametrize("T,N", [(1, 8), (31, 136), (33, 1152), (9000, 4608), (5, 20)])
+def test_column_sums(T, N):
+    torch.manual_seed(0)
+    x = torch.randn(T, N, device=DEV).to(torch.bfloat16)
+    out = torch.randn(N, device=DEV)
+    want = out.double() + x.double().sum(0)
+    torch.testing.assert_close(dense._column_sums(x, out).double(), want, rtol=1e-5, atol=1e-4 * T ** 0.5)
+    torch.testing.assert_close(dense._column_sums(x).double(), x.double().sum(0), rtol=1e-5, atol=1e-4 * T ** 0.5)
+
+
+@pytest.mark.parametrize("T,H", [(1, 8), (700, 896), (595, 1024), (300, 1032), (40, 3584), (2500, 64)])
+def test_rmsnorm_backward_widths(T, H):
+    """Both block widths, more rows than blocks and fewer."""
+    torch.manual_seed(0)
+    x, r = (torch.randn(T, H, device=DEV).to(torch.bfloat16).requires_grad_() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, device=DEV)).to(torch.bfloat16).requires_grad_()
+    y, h = ops.rmsnorm(x, w, 1e-6, residual=r)
+    gy, gh = torch.randn_like(y), torch.randn_like(h)
+    torch.autograd.backward([y, h], [gy, gh])
+    hd, wd = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    yd = hd * torch.rsqrt(hd.square().mean(-1, keepdim=True) + 1e-6) * wd
+    torch.autograd.backward([yd], [gy.double()])
+    want = hd.grad + gh.double()
+    # one rounding to bf16 (2^-9 relative); the weight's gradient is rounded after a 32-bit sum
+    assert ((x.grad.double() - want).norm() / want.norm()).item() < 3e-3 and torch.equal(x.grad, r.grad)
+    assert ((w.grad.double() - wd.grad).norm() / wd.grad.norm()).item() < 4e-3

@@ -57,7 +57,7 @@ __device__ __forceinline__ void adamw_element(const AdamParams& p, float gs, flo
 // and marks them as read once, so that they do not push the weights out of L2; one element per thread kept only 32 KB
 // per SM in flight.  A block's piece is contiguous and small (64 blocks per SM): eight streams at distances that change with
 // every block spread better over the memory than in lockstep sweeps.  512 M parameters: one element per thread 5.28 ms (3.0
-// TB/s); 16 bytes in sweeps of 8 blocks per SM 3.55 ms, of 64 3.24 ms; in pieces 3.16 ms (5.1 TB/s).
+// TB/s); 16 bytes in sweeps of 8 blocks per SM 3.55 ms, of 64 3.24 ms; in pieces 3.21 ms (5.0 TB/s).
 // VEC = 1 serves shards whose start is no multiple of four elements, and the last n % 4 elements.
 template <int VEC>
 __global__ void __launch_bounds__(256) adamw_kernel(AdamParams p) {

@@ -10,16 +10,25 @@
 //   dQ_i is added to an fp32 buffer by vector reductions of whole 128-byte lines
 // The softmax scale is applied once, to dK and dQ at the end.
 //
+// Blocks that share a group's heads keep dK and dV apart for the pass that converts them, which adds them in order.  dQ comes
+// from all K/V tiles of a sequence.  ORDERED: they add to it one after the other, tile 0 first (it stores, nothing is
+// zeroed), so that equal inputs give equal gradients.  Tiles then walk over the query tiles from the last to the first and
+// take their work by ticket, tile 0 first: no block waits for one that may not have started, and the one it waits for is
+// ahead unless both start at once.  Else tiles start on the diagonal and add as they come: tiles that run together are then
+// always at different rows, and none waits until its predecessor's additions have reached memory.  Microseconds ordered /
+// not, causal: 8 x 568-1232, 14 / 2 heads, D = 64: 144 / 142; 4 x 1024, 28 / 4, D = 128: 230 / 206; 8 x 2048: 1088 / 873;
+// 1 x 4096: 551 / 398; 1 x 16384: 7430 / 5500; 1 x 9900, 14 / 2, D = 64: 955 / 713.
+//
 // What bounds it: the five products take 2560 cycles a step with D = 128 (1536 with D = 64, whose operands come from shared
 // memory at its full rate), the exponentials 1024 and the rest of the element-wise work about as much.  All of it is in
 // flight at once: while the math warps take step i + 1 from scores to weights the tensor cores run dQ, dK and dP behind
 // step i, and while they go from dP to dS, dV and the next scores.  Lane = kv row because P^T is then an operand in TMEM
 // (no shared memory, which is full with D = 128); the row statistics become columns, staged by a warp of their own.
-// Blocks are ordered by their number of steps.  One block per kv head leaves SMs idle when a sequence is long and kv heads
+// Blocks are listed by their number of steps.  One block per kv head leaves SMs idle when a sequence is long and kv heads
 // are few: its first K/V tile has twice the average work, times the heads of the group.  The caller then splits the group
 // (bwd_head_splits).  Causal, before (256 threads, one step after the other) and now: 28 / 4 heads, D = 128, 1 x 16384:
-// 9.99 ms (482 TFLOP/s), 5.00 ms (962); 8 x 2048: 1.49 ms, 0.86 ms; 14 / 2 heads, D = 64, 1 x 9900: 2.24 ms (196), 0.72 ms
-// (608; unsplit 1.21 ms); 8 x 500-1550: 0.38 ms, 0.15 ms (unsplit 0.24 ms).
+// 9.99 ms (482 TFLOP/s), 5.50 ms (875); 8 x 2048: 1.50 ms, 1.09 ms; 14 / 2 heads, D = 64, 1 x 9900: 2.15 ms (204), 0.71 ms
+// (617; unsplit 1.21 ms); 8 x 568-1232: 0.31 ms, 0.14 ms (unsplit 0.24 ms).
 #include "common.cuh"
 #include "launchers.h"
 
@@ -31,8 +40,10 @@ struct FmhaBwdParams {
   const int* tile_k0;         // first kv position of the tile inside its sequence
   const float* lse;           // [Hq, T]
   const float* delta;         // [Hq, T]  rowsum(dO * O)
-  float* dq_accum;            // [T, Hq*D] fp32, zero-initialised
-  float* dkv_accum;           // [T, 2*Hkv*D] fp32, zero-initialised, when the q heads of a group are split (else unused)
+  float* dq_accum;            // [T, Hq*D] fp32, zero-initialised when the tiles are not ordered
+  float* dkv_accum;           // [head_splits, T, 2*Hkv*D] fp32 when the q heads of a group are split (else unused)
+  int* turn;                  // ordered: [Hq, T + 1] zero-initialised: at the first of each 32 query rows of a sequence the
+                              // number of K/V tiles that have added their dQ; at row T of head 0 the next block's ticket
   __nv_bfloat16* dqkv;        // [T, (Hq+2Hkv)*D]; this kernel writes the k and v parts when they are not split
   int T, Hq, Hkv, causal, head_splits;
   float scale, scale_log2;
@@ -55,7 +66,7 @@ struct BwdSmem {
   static constexpr int kStageOff = kDsOff + kSq;
   static constexpr int kStatOff = kStageOff + 128 * kBwdStagePitch;  // 2 x (128 of -lse * log2e, 128 of -delta)
   static constexpr int kBarOff = kStatOff + 2 * 1024;
-  static constexpr int kTotal = kBarOff + 20 * 8 + 16;
+  static constexpr int kTotal = kBarOff + 20 * 8 + 16;  // barriers, TMEM address, ticket
   static_assert(2 * 128 * kAccPitch <= kStageOff, "dK and dV rows are staged over the operand tiles");
 };
 
@@ -64,11 +75,42 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
                : "memory");
 }
 
-// adds `bytes` bytes of fp32 from shared memory to global memory (both 16-byte aligned)
-__device__ __forceinline__ void bulk_add_f32(float* dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
-               "r"(bytes)
+// copies `bytes` bytes from shared memory to global memory (both 16-byte aligned)
+__device__ __forceinline__ void bulk_store(float* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
                : "memory");
+}
+
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {  // returns at once
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// Bounded wait until *turn, written by other blocks of this kernel, is at least `n`.
+__device__ __forceinline__ bool wait_turn(const int* turn, int n, int* status) {
+  auto arrived = [&] {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(turn) : "memory");
+    return v >= n;
+  };
+  if (arrived()) return true;
+  const uint64_t t0 = global_timer_ns();
+  while (true) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (arrived()) return true;
+    if (global_timer_ns() - t0 > SB_WAIT_LIMIT_NS) {
+      atomicCAS(status, 0, (int)kStatusTimeoutFlag);
+      return false;
+    }
+  }
 }
 
 template <int N>
@@ -103,7 +145,7 @@ constexpr int kBwdThreads = 512;
 constexpr int kRegsMath = 144, kRegsDq = 152, kRegsIssue = 72;
 static_assert(2 * kRegsMath + kRegsDq + kRegsIssue <= 4 * 128, "more registers than the launch has");
 
-template <int D>
+template <int D, bool ORDERED>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_do,
                 FmhaBwdParams p) {
@@ -136,19 +178,22 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
   uint64_t* dq_read = bar_kv + 18;
   uint64_t* done = bar_kv + 19;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_kv + 20);
+  int* ticket_slot = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per_tile = p.Hkv * p.head_splits;
-  const int tile = (int)(blockIdx.x / per_tile), kvh = (int)(blockIdx.x % per_tile) / p.head_splits;
-  const int share = (int)(blockIdx.x % per_tile) % p.head_splits;
-  const int seq_start = p.tile_seq_start[tile], seq_len = p.tile_seq_len[tile], k0 = p.tile_k0[tile];
-  const int rep = p.Hq / p.Hkv;
-  const int h_first = kvh * rep + rep * share / p.head_splits, h_end = kvh * rep + rep * (share + 1) / p.head_splits;
-  const int i_start = p.causal ? (k0 / 128) : 0;
-  const int per_head = (seq_len + 127) / 128 - i_start;
-  const int steps = per_head * (h_end - h_first);
-  const int kcol = (p.Hq + kvh) * D, vcol = (p.Hq + p.Hkv + kvh) * D;
-
+  int ticket = (int)blockIdx.x, seq_start, seq_len, k0;
+  auto take_tile = [&] {
+    const int tile = ticket / per_tile;
+    seq_start = p.tile_seq_start[tile];
+    seq_len = p.tile_seq_len[tile];
+    k0 = p.tile_k0[tile];
+  };
+  if (ORDERED) {
+    if (tid == 32) *ticket_slot = atomicAdd(p.turn + p.T, 1);
+  } else {
+    take_tile();
+  }
   if (tid == 0) {
     tma_prefetch_desc(&map_qkv);
     tma_prefetch_desc(&map_do);
@@ -170,6 +215,19 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
   const uint32_t tm_dq = kDqOverDp ? tm_dp : tm_dk + D;
   const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
 
+  if (ORDERED) {
+    ticket = *ticket_slot;
+    take_tile();
+  }
+  const int kvh = ticket % per_tile / p.head_splits, share = ticket % per_tile % p.head_splits;
+  const int rep = p.Hq / p.Hkv;
+  const int h_first = kvh * rep + rep * share / p.head_splits, h_end = kvh * rep + rep * (share + 1) / p.head_splits;
+  const int i_low = p.causal ? k0 / 128 : 0, i_high = (seq_len + 127) / 128 - 1, per_head = i_high + 1 - i_low;
+  const int i_first = ORDERED ? i_high : i_low;  // query tiles of every head: from here down, or up
+  constexpr int kDir = ORDERED ? -1 : 1;
+  const int steps = per_head * (h_end - h_first);
+  const int kcol = (p.Hq + kvh) * D, vcol = (p.Hq + p.Hkv + kvh) * D;
+
   if (warp < 8) {
     // ------------------------------ P and dS, then dK and dV ------------------------------
     regs_inc<kRegsMath>();
@@ -177,7 +235,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
     const int kp = k0 + r;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
-    int q0 = i_start * 128, left = per_head;
+    int q0 = i_first * 128, left = per_head;
     for (int i = 0; i < steps; ++i) {
       const float4* stat = reinterpret_cast<const float4*>(smem + L::kStatOff + (i & 1) * 1024) + half * 16;
       ok = __all_sync(0xffffffffu, mbar_wait(&st_full[i & 1], (i >> 1) & 1, p.status, kStatusTimeoutEpilogue) &&
@@ -246,10 +304,10 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
       tc_fence_before();
       mbar_arrive(ds_ready);
       mbar_arrive(&st_empty[i & 1]);
-      q0 += 128;
+      q0 += kDir * 128;
       if (--left == 0) {
         left = per_head;
-        q0 = i_start * 128;
+        q0 = i_first * 128;
       }
     }
     // ---- dK, dV (lane = kv row, this warp's half of the D columns) ----
@@ -267,7 +325,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
         tmem_ld_32x32((is_v ? tm_dv : tm_dk) + lane_off + col, ra);
         tmem_ld_wait();
         if (p.head_splits > 1) {
-          // every MMA has read its operands: their tiles hold the rows on the way to the fp32 sums of the group
+          // every MMA has read its operands: their tiles hold the rows on the way to this share's fp32 sums
           float* stage = reinterpret_cast<float*>(smem + (is_v * 128 + r) * L::kAccPitch) + col;
 #pragma unroll
           for (int g = 0; g < 8; ++g)
@@ -276,7 +334,8 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
                             __uint_as_float(ra[g * 4 + 2]) * f, __uint_as_float(ra[g * 4 + 3]) * f);
           fence_proxy_async_smem();
           if (row_valid)
-            bulk_add_f32(p.dkv_accum + row * (size_t)(2 * p.Hkv * D) + (size_t)((is_v ? p.Hkv : 0) + kvh) * D + col, stage, 128);
+            bulk_store(p.dkv_accum + ((size_t)share * p.T + row) * (size_t)(2 * p.Hkv * D) +
+                           (size_t)((is_v ? p.Hkv : 0) + kvh) * D + col, stage, 128);
           tma_store_commit();
         } else if (row_valid) {
           __nv_bfloat16* dst = p.dqkv + row * (size_t)((p.Hq + 2 * p.Hkv) * D) + (is_v ? vcol : kcol) + col;
@@ -297,7 +356,15 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
     // ------------------------------ dQ -> fp32 sums (lane = query row) ------------------------------
     regs_inc<kRegsDq>();
     uint8_t* stage = smem + L::kStageOff + (warp & 3) * (32 * kBwdStagePitch);
-    int q0 = i_start * 128, left = per_head, h = h_first;
+    const int order = k0 / 128;   // of this tile among those that add to a query tile
+    int* next = nullptr;          // where the tile behind this one waits for the previous step's rows
+    auto hand_on = [&] {
+      if (next == nullptr) return;
+      __syncwarp();
+      if (lane == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(next), "r"(order + 1) : "memory");
+      next = nullptr;
+    };
+    int q0 = i_first * 128, left = per_head, h = h_first;
     for (int i = 0; i < steps; ++i) {
       if (!__all_sync(0xffffffffu, mbar_wait(dq_full, i & 1, p.status, kStatusTimeoutEpilogue))) break;
       tc_fence_after();
@@ -307,9 +374,16 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(dq_read);
+      if (ORDERED) hand_on();
+      const int first = q0 + (warp & 3) * 32;
+      int* turn = ORDERED ? p.turn + (size_t)h * (p.T + 1) + seq_start + first : nullptr;
+      if (ORDERED && first < seq_len && order > 0) {
+        bool mine = true;
+        if (lane == 0) mine = wait_turn(turn, order, p.status);
+        if (!__all_sync(0xffffffffu, mine)) break;
+      }
       // TMEM hands every thread one query row; turned through shared memory, each warp instruction adds four lines of
       // 128 bytes instead of 32 pieces of 16
-      const int first = q0 + (warp & 3) * 32;
       float* dst = p.dq_accum + (size_t)(seq_start + first) * (size_t)(p.Hq * D) + (size_t)h * D + (lane & 7) * 4;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
@@ -322,14 +396,24 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
         for (int g = 0; g < 8; ++g) {
           const int row = g * 4 + (lane >> 3);
           const float4 v = *reinterpret_cast<const float4*>(stage + row * kBwdStagePitch + (lane & 7) * 16);
-          if (first + row < seq_len) red_add_v4(dst + (size_t)row * (size_t)(p.Hq * D) + c * 32, v.x, v.y, v.z, v.w);
+          float* at = dst + (size_t)row * (size_t)(p.Hq * D) + c * 32;
+          if (first + row < seq_len) {
+            if (ORDERED && order == 0) *reinterpret_cast<float4*>(at) = v;
+            else red_add_v4(at, v.x, v.y, v.z, v.w);
+          }
         }
         __syncwarp();
       }
-      q0 += 128;
+      if (ORDERED) {
+        // Rows are handed on at once while there is nothing else to do, else behind the next step's loads: by then the
+        // additions are done, and the release does not wait for them.
+        if (first < seq_len && order < (p.causal ? q0 / 128 : i_high)) next = turn;
+        if (i + 1 == steps || !__all_sync(0xffffffffu, mbar_test(dq_full, (i + 1) & 1))) hand_on();
+      }
+      q0 += kDir * 128;
       if (--left == 0) {
         left = per_head;
-        q0 = i_start * 128;
+        q0 = i_first * 128;
         ++h;
       }
     }
@@ -345,7 +429,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
           tma_load_2d(sV + c * 16384, &map_qkv, bar_kv, vcol + c * 64, seq_start + k0);
         }
         int n_q = 0, n_do = 0;  // loads issued
-        int qi = i_start, left = per_head, h = h_first;
+        int qi = i_first, left = per_head, h = h_first;
         for (int i = 0; i < steps; ++i) {
           const int row = seq_start + qi * 128;
           if (!mbar_wait(&q_empty[i & 1], ((i >> 1) & 1) ^ 1, p.status, kStatusTimeoutProducer)) break;
@@ -360,10 +444,10 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
           for (int c = 0; c < kDChunks; ++c)
             tma_load_2d(sDo + (i % kDo) * L::kTile + c * 16384, &map_do, &do_full[i % kDo], h * D + c * 64, row);
           n_do = i + 1;
-          ++qi;
+          qi += kDir;
           if (--left == 0) {
             left = per_head;
-            qi = i_start;
+            qi = i_first;
             ++h;
           }
         }
@@ -440,7 +524,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
       umma_commit_if(leader, done);
     } else if (warp == 14) {
       // ------------------------------ row statistics: -lse * log2(e), -delta ------------------------------
-      int q0 = i_start * 128, left = per_head, h = h_first;
+      int q0 = i_first * 128, left = per_head, h = h_first;
       for (int i = 0; i < steps; ++i) {
         if (!__all_sync(0xffffffffu, mbar_wait(&st_empty[i & 1], ((i >> 1) & 1) ^ 1, p.status, kStatusTimeoutProducer))) break;
         float* dst = reinterpret_cast<float*>(smem + L::kStatOff + (i & 1) * 1024);
@@ -453,10 +537,10 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
           dst[128 + q] = in ? -p.delta[at + q] : 0.f;
         }
         mbar_arrive(&st_full[i & 1]);
-        q0 += 128;
+        q0 += kDir * 128;
         if (--left == 0) {
           left = per_head;
-          q0 = i_start * 128;
+          q0 = i_first * 128;
           ++h;
         }
       }
@@ -470,9 +554,9 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
   }
 }
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h)
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h).  Clears `turn` as well (if not null).
 __global__ void fmha_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  float* __restrict__ delta, int T, int Hq, int D) {
+                                  float* __restrict__ delta, int* __restrict__ turn, int T, int Hq, int D) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= (long long)T * Hq) return;
@@ -486,17 +570,28 @@ __global__ void fmha_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
     s += x.x * y.x + x.y * y.y;
   }
   s = warp_sum(s);
-  if (lane == 0) delta[(size_t)h * T + t] = s;
+  if (lane == 0) {
+    delta[(size_t)h * T + t] = s;
+    if (turn) {
+      turn[(size_t)h * (T + 1) + t] = 0;
+      if (t == 0) turn[(size_t)h * (T + 1) + T] = 0;
+    }
+  }
 }
 
-// dqkv[t, col + c] = bf16(acc[t, c] * scale) for `cols` columns
-__global__ void fmha_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv, int T, int cols, int col,
-                                 int width, float scale) {
+// dqkv[t, col + c] = bf16(scale * acc[t, c]) for `cols` columns; SUM: of the sum of `slabs` such buffers
+template <bool SUM>
+__global__ void fmha_cast_kernel(const float* __restrict__ acc, int slabs, __nv_bfloat16* __restrict__ dqkv, int T, int cols,
+                                 int col, int width, float scale) {
   const long long total = (long long)T * (cols / 4);
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const int t = (int)(idx / (cols / 4)), c = (int)(idx % (cols / 4)) * 4;
-    const float4 v = *reinterpret_cast<const float4*>(acc + (size_t)t * cols + c);
+    float4 v = *reinterpret_cast<const float4*>(acc + (size_t)t * cols + c);
+    for (int s = 1; SUM && s < slabs; ++s) {
+      const float4 b = *reinterpret_cast<const float4*>(acc + ((size_t)s * T + t) * cols + c);
+      v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+    }
     uint2 o;
     o.x = pack_bf16x2(v.x * scale, v.y * scale);
     o.y = pack_bf16x2(v.z * scale, v.w * scale);
@@ -504,18 +599,19 @@ __global__ void fmha_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* _
   }
 }
 
-static void launch_cast(const float* acc, __nv_bfloat16* dqkv, int T, int cols, int col, int width, float scale,
+static void launch_cast(const float* acc, int slabs, __nv_bfloat16* dqkv, int T, int cols, int col, int width, float scale,
                         cudaStream_t stream) {
   const long long total = (long long)T * (cols / 4), cap = (long long)num_sms() * 8;
   const long long blocks = (total + 255) / 256;
-  fmha_cast_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, stream>>>(acc, dqkv, T, cols, col, width, scale);
+  auto kernel = slabs > 1 ? fmha_cast_kernel<true> : fmha_cast_kernel<false>;
+  kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, stream>>>(acc, slabs, dqkv, T, cols, col, width, scale);
 }
 
-template <int D>
+template <int D, bool ORDERED>
 static int launch_bwd(const CUtensorMap& mqkv, const CUtensorMap& mdo, const FmhaBwdParams& p, int num_tiles,
                       cudaStream_t stream) {
   using L = BwdSmem<D>;
-  auto kernel = fmha_bwd_kernel<D>;
+  auto kernel = fmha_bwd_kernel<D, ORDERED>;
   static bool configured = false;
   if (!configured) {
     cudaFuncAttributes attr;
@@ -537,11 +633,12 @@ static int launch_bwd(const CUtensorMap& mqkv, const CUtensorMap& mdo, const Fmh
 
 using namespace sb;
 
-// qkv: packed forward input; out/d_out: [T, Hq*D]; dq_accum: fp32 scratch [T, Hq*D] (zeroed here);
-// delta: fp32 scratch [Hq, T]; dqkv: packed gradient output.  head_splits > 1 divides the q heads of each group over that
-// many blocks, whose dK and dV meet in dkv_accum: fp32 scratch [T, 2*Hkv*D] (zeroed here).
+// qkv: packed forward input; out/d_out: [T, Hq*D]; dq_accum: fp32 scratch [T, Hq*D]; delta: fp32 scratch [Hq, T]; dqkv: packed
+// gradient output.  head_splits > 1 divides the q heads of each group over that many blocks, whose dK and dV go to dkv_accum:
+// fp32 scratch [head_splits, T, 2*Hkv*D].  turn: int scratch [Hq, T + 1] for ordered sums, or null.  For these all tiles of a
+// sequence stand in the lists, tile_k0 ascending, and rows outside the sequences get what dq_accum holds as their q gradient.
 extern "C" int sb_fmha_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,
-                           float* dq_accum, float* dkv_accum, void* dqkv, const int* tile_seq_start,
+                           float* dq_accum, float* dkv_accum, int* turn, void* dqkv, const int* tile_seq_start,
                            const int* tile_seq_len, const int* tile_k0, int num_tiles, int T, int Hq, int Hkv, int D,
                            int causal, int head_splits, float scale, int* status, cudaStream_t stream) {
   if (num_tiles == 0 || T == 0) return 0;
@@ -559,25 +656,25 @@ extern "C" int sb_fmha_bwd(const void* qkv, const void* out, const void* d_out, 
   if (r) return r;
   r = make_tensor_map_bf16_2d(&mdo, d_out, qwidth, T, qwidth, 64, 128);
   if (r) return r;
-  cudaMemsetAsync(dq_accum, 0, sizeof(float) * (size_t)T * qwidth, stream);
-  if (head_splits > 1) cudaMemsetAsync(dkv_accum, 0, sizeof(float) * (size_t)T * 2 * Hkv * D, stream);
+  if (!turn) cudaMemsetAsync(dq_accum, 0, sizeof(float) * (size_t)T * qwidth, stream);
   {
     const long long warps = (long long)T * Hq;
     const int threads = 256;
     const long long blocks = (warps * 32 + threads - 1) / threads;
     fmha_delta_kernel<<<(unsigned)blocks, threads, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out,
-                                                                delta, T, Hq, D);
+                                                                delta, turn, T, Hq, D);
   }
   FmhaBwdParams p;
   p.tile_seq_start = tile_seq_start; p.tile_seq_len = tile_seq_len; p.tile_k0 = tile_k0;
-  p.lse = lse; p.delta = delta; p.dq_accum = dq_accum; p.dkv_accum = dkv_accum;
+  p.lse = lse; p.delta = delta; p.dq_accum = dq_accum; p.dkv_accum = dkv_accum; p.turn = turn;
   p.dqkv = reinterpret_cast<__nv_bfloat16*>(dqkv);
   p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal; p.head_splits = head_splits;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  r = (D == 128) ? launch_bwd<128>(mqkv, mdo, p, num_tiles, stream) : launch_bwd<64>(mqkv, mdo, p, num_tiles, stream);
+  if (turn) r = D == 128 ? launch_bwd<128, true>(mqkv, mdo, p, num_tiles, stream) : launch_bwd<64, true>(mqkv, mdo, p, num_tiles, stream);
+  else r = D == 128 ? launch_bwd<128, false>(mqkv, mdo, p, num_tiles, stream) : launch_bwd<64, false>(mqkv, mdo, p, num_tiles, stream);
   if (r) return r;
-  launch_cast(dq_accum, p.dqkv, T, (int)qwidth, 0, (int)width, scale, stream);
-  if (head_splits > 1) launch_cast(dkv_accum, p.dqkv, T, 2 * Hkv * D, (int)qwidth, (int)width, 1.f, stream);
+  launch_cast(dq_accum, 1, p.dqkv, T, (int)qwidth, 0, (int)width, scale, stream);
+  if (head_splits > 1) launch_cast(dkv_accum, head_splits, p.dqkv, T, 2 * Hkv * D, (int)qwidth, (int)width, 1.f, stream);
   return (int)cudaGetLastError();
 }

@@ -104,7 +104,7 @@ int sb_fmha_fwd(const void* qkv, void* out, float* lse, const int* tile_seq_star
                 const int* tile_q0, int num_tiles, int T, int Hq, int Hkv, int D, int causal, float scale,
                 int* status, cudaStream_t stream);
 int sb_fmha_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,
-                float* dq_accum, float* dkv_accum, void* dqkv, const int* tile_seq_start, const int* tile_seq_len,
+                float* dq_accum, float* dkv_accum, int* turn, void* dqkv, const int* tile_seq_start, const int* tile_seq_len,
                 const int* tile_k0, int num_tiles, int T, int Hq, int Hkv, int D, int causal, int head_splits,
                 float scale, int* status, cudaStream_t stream);
 }

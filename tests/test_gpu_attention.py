@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from siirl_b200.ops import lib, reference as ref
-from siirl_b200.ops.attention import SeqInfo, attention_packed, bwd_head_splits
+from siirl_b200.ops.attention import SeqInfo, attention_packed, bwd_head_splits, bwd_ordered
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -110,3 +110,48 @@ def test_attention_bwd_tiles(d, hq, hkv, repeat, splits, causal):
         # P, dS and the results are rounded to bf16 (2^-9 each): 2.5e-3 measured over these sizes, four times that allowed
         assert _rel(got[:, a:b], x.grad[:, a:b]) < 1e-2
     assert torch.isfinite(qkv.grad.float()).all()
+
+
+@pytest.mark.parametrize("d,hq,hkv,seqlens,causal", [
+    (64, 14, 2, [904, 1232, 33, 568], True), (128, 6, 2, [1500, 130], True), (64, 4, 4, [600] * 80, True),
+    (128, 7, 1, [4000], True), (64, 14, 2, [4097, 129], True), (128, 28, 4, [300, 500, 1550], False)])
+def test_attention_bwd_repeats_itself(d, hq, hkv, seqlens, causal):
+    """Equal inputs give equal gradients, bit by bit, however the blocks are scheduled: with the heads of a group in one
+    block and divided, fewer blocks than SMs and several waves, alone and beside other work.  Causal sequences of up to
+    64 d rows do so by themselves, the last two cases when torch asks for it."""
+    torch.manual_seed(3)
+    T = sum(seqlens)
+    assert bwd_ordered(max(seqlens), d, causal) == (causal and max(seqlens) <= 4096)
+    info = SeqInfo(seqlens, device=DEV)
+    qkv = torch.randn(T, (hq + 2 * hkv) * d, device=DEV).to(torch.bfloat16).requires_grad_()
+    out = attention_packed(qkv, info, hq, hkv, d, causal=causal)
+    g = torch.randn_like(out)
+    side, busy = torch.cuda.Stream(), torch.randn(1 << 22, device=DEV)
+    torch.use_deterministic_algorithms(not bwd_ordered(max(seqlens), d, causal))
+    try:
+        want, = torch.autograd.grad(out, qkv, g, retain_graph=True)
+        for i in range(6):
+            if i % 2:
+                side.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(side):
+                    for _ in range(20):
+                        busy.mul_(1.0)
+            got, = torch.autograd.grad(out, qkv, g, retain_graph=True)
+            assert torch.equal(got, want), i
+    finally:
+        torch.use_deterministic_algorithms(False)
+    torch.cuda.synchronize()
+    lib.check_status()
+    # the same sums in the other order: fp32 rounding moves a few results to the next bf16 number
+    torch.testing.assert_close(want, _other_order(qkv, info, out, g, hq, hkv, d, causal), rtol=2 ** -6, atol=1e-3)
+
+
+def _other_order(qkv, info, out, g, hq, hkv, d, causal):
+    """The gradient with one block per kv head and unordered sums of dQ."""
+    from siirl_b200.ops import attention as att
+    keep = att.bwd_ordered, att.bwd_head_splits
+    att.bwd_ordered, att.bwd_head_splits = lambda *a: False, lambda *a: 1
+    try:
+        return torch.autograd.grad(out, qkv, g)[0]
+    finally:
+        att.bwd_ordered, att.bwd_head_splits = keep

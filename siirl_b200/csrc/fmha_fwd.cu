@@ -4,7 +4,7 @@
 // siirl/models/transformers/monkey_patch.py:51-109).
 //
 // Layout: one packed buffer qkv[T, (Hq + 2*Hkv) * D] (q heads, then k heads, then v heads per row);
-// sequences are row ranges given by cu_seqlens.  One CTA = 256 query rows (two 128-row tiles) of one q head:
+// sequences are row ranges given by cu_seqlens.  One CTA = 256 query rows (two 128-row tiles) of one q head, or 128:
 //   S_w = Q_w K_j^T     tcgen05.mma 128 x KV x D    -> TMEM, w = 0, 1
 //   softmax             one warpgroup per query tile, thread = row; the weights (bf16) replace the scores in TMEM
 //   O_w += P_w V_j      tcgen05.mma 128 x D x KV, P from TMEM, V through an MN-major descriptor (no transpose copy)
@@ -18,7 +18,9 @@
 // for 128 keys and one CTA (14 / 2 heads, sequences of 14900 and 15400).  Causal, before (one 128-row tile per CTA, each step
 // waiting for the one before) and now: D = 128, 28 / 4 heads, 1 x 16384: 3.47 ms (554 TFLOP/s), 1.85 ms (1045); 8 x 2048:
 // 0.56 ms, 0.37 ms; D = 64, 14 / 2 heads, the sequences above: 1.95 ms (423), 1.14 ms (720).  Short sequences are bound by
-// the latency of a CTA's first loads, softmax and stores, some 7 us: 32 x 256-1000 tokens, D = 128: 0.36 ms, 0.32 ms.
+// the latency of a CTA's first loads, softmax and stores, some 7 us: 32 x 256-1000 tokens, D = 128: 0.36 ms, 0.32 ms.  With
+// one tile and 64 keys at a time two CTAs (D = 128) or three fit an SM: 128 x 128 tokens, 28 / 4 heads, D = 128: 133 us
+// (one tile per CTA, each step waiting for the one before), 188 (two tiles), 119; D = 64, 14 / 2: 38, 43, 35.
 #include "common.cuh"
 #include "launchers.h"
 
@@ -36,12 +38,12 @@ struct FmhaFwdParams {
   int* status;
 };
 
-template <int D, int KV>
+template <int D, int KV, int QT>
 struct FwdSmem {
-  static constexpr int kQBytes = 128 * D * 2;   // one of the two query tiles
+  static constexpr int kQBytes = 128 * D * 2;   // one query tile
   static constexpr int kKvBytes = KV * D * 2;   // one K or V tile
-  static constexpr int kStages = D == 128 ? 5 : 6;
-  static constexpr int kRingOff = 2 * kQBytes;
+  static constexpr int kStages = QT == 1 ? 4 : D == 128 ? 5 : 6;
+  static constexpr int kRingOff = QT * kQBytes;
   static constexpr int kBarOff = kRingOff + kStages * kKvBytes;  // q[2], s_full[2], p_full[2], o_full[2], full[], empty[]
   static constexpr int kTotal = kBarOff + (8 + 2 * kStages) * 8 + 16;
 };
@@ -60,15 +62,16 @@ __device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
   return *reinterpret_cast<float2*>(&d);
 }
 
-// KV: keys of a tile; CTAS: blocks of an SM.
-// Warps 0-3 and 4-7: softmax of query tile 0 and 1 (thread = row); warp 8: TMA; warp 9: MMA issuer.
-template <int D, int KV, int CTAS>
-__global__ void __launch_bounds__(320, CTAS)
+// KV: keys of a tile; QT: query tiles; CTAS: blocks of an SM.
+// Four warps for the softmax of each query tile (thread = row), then one for TMA and the MMA issuer.
+template <int D, int KV, int QT, int CTAS>
+__global__ void __launch_bounds__(QT * 128 + 64, CTAS)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                 FmhaFwdParams p) {
-  using L = FwdSmem<D, KV>;
-  constexpr int kDChunks = D / 64, kStages = L::kStages;
-  constexpr uint32_t kTmemCols = (2 * (KV + D) <= 256) ? 256 : 512;  // S (P over it) and O of both tiles
+  using L = FwdSmem<D, KV, QT>;
+  constexpr int kDChunks = D / 64, kStages = L::kStages, kTmaWarp = QT * 4, kMmaWarp = QT * 4 + 1;
+  // S (P over it) and O of every query tile
+  constexpr uint32_t kTmemCols = QT * (KV + D) <= 128 ? 128 : QT * (KV + D) <= 256 ? 256 : 512;
   // 1024-byte alignment is required by the 128-byte swizzle
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
@@ -94,7 +97,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     for (int i = 0; i < 2 * kStages; ++i) mbar_init(&full[i], 1);
     fence_barrier_init();
   }
-  if (warp == 9) {
+  if (warp == kMmaWarp) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
@@ -112,10 +115,10 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (first >= seq_len) return 0;
     return ((p.causal ? min(first + 128, seq_len) : seq_len) + KV - 1) / KV;
   };
-  const int n0 = key_tiles(0), n1 = key_tiles(1);
+  const int n0 = key_tiles(0), n1 = QT == 2 ? key_tiles(1) : 0;
   const int n_max = max(n0, n1);
 
-  if (warp == 8) {
+  if (warp == kTmaWarp) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
       const int qcol = h * D, kcol = (p.Hq + kvh) * D, vcol = (p.Hq + p.Hkv + kvh) * D;
@@ -143,7 +146,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         for (int k = max(0, i - kStages); k < i; ++k) mbar_wait(&full[k % kStages], (k / kStages) & 1, nullptr, 0);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issuer (converged; lane 0 issues) ------------------------------
     constexpr uint32_t idesc_s = umma_idesc_bf16(128, KV, 0, 0);
     constexpr uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
@@ -176,7 +179,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     for (int j = 0; j < n_max && ok; ++j) {
       ok = wait_ring(2 * j + 1);
 #pragma unroll
-      for (int w = 0; w < 2; ++w) {
+      for (int w = 0; w < QT; ++w) {
         const int n = w ? n1 : n0;
         if (ok && j < n) {
           ok = wait(&p_full[w], j & 1);
@@ -184,12 +187,12 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const uint32_t bv = ar + ((2 * j + 1) % kStages) * L::kKvBytes;
 #pragma unroll
             for (int kk = 0; kk < KV / 16; ++kk)
-              umma_bf16_ts_if(leader, tmem_base + 2 * KV + w * D, tmem_base + w * KV + kk * 8,
+              umma_bf16_ts_if(leader, tmem_base + QT * KV + w * D, tmem_base + w * KV + kk * 8,
                               umma_smem_desc(bv + kk * 2048, KV * 128, 1024), idesc_o, (j | kk) ? 1u : 0u);
             if (j + 1 == n) umma_commit_if(leader, &o_full[w]);
           }
         }
-        if (w == 1) umma_commit_if(leader, &empty[(2 * j + 1) % kStages]);
+        if (w == QT - 1) umma_commit_if(leader, &empty[(2 * j + 1) % kStages]);
         if (ok && j + 1 < n) {
           ok = wait_ring(2 * j + 2);
           if (ok) scores(w, j + 1);
@@ -202,7 +205,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int w = warp >> 2;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tmem_s = tmem_base + lane_off + w * KV;
-    const uint32_t tmem_o = tmem_base + lane_off + 2 * KV + w * D;
+    const uint32_t tmem_o = tmem_base + lane_off + QT * KV + w * D;
     const int first = q0 + w * 128;
     const int qpos = first + (warp & 3) * 32 + lane;  // position within the sequence
     const int n = w ? n1 : n0;
@@ -309,17 +312,17 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
-template <int D, int KV, int CTAS>
+template <int D, int KV, int QT, int CTAS>
 static int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mkv, const FmhaFwdParams& p, int num_tiles,
                       cudaStream_t stream) {
-  using L = FwdSmem<D, KV>;
-  auto kernel = fmha_fwd_kernel<D, KV, CTAS>;
+  using L = FwdSmem<D, KV, QT>;
+  auto kernel = fmha_fwd_kernel<D, KV, QT, CTAS>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
@@ -328,19 +331,21 @@ static int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mkv, const FmhaF
   }
   const long long blocks = (long long)num_tiles * p.Hq;
   if (blocks > 0x7fffffffll) return -4;
-  return launch_chained(kernel, (unsigned)blocks, 320, L::kTotal, stream, mq, mkv, p);
+  return launch_chained(kernel, (unsigned)blocks, QT * 128 + 64, L::kTotal, stream, mq, mkv, p);
 }
 
 }  // namespace sb
 
 using namespace sb;
 
-// Tiles are 256 query rows: entry i covers rows tile_q0[i] .. tile_q0[i] + 255 (as far as they exist) of its sequence.
+// Entry i of the tile lists covers tile_rows (128 or 256) query rows from tile_q0[i] on, as far as they exist, of its
+// sequence.
 extern "C" int sb_fmha_fwd(const void* qkv, void* out, float* lse, const int* tile_seq_start,
-                           const int* tile_seq_len, const int* tile_q0, int num_tiles, int T, int Hq, int Hkv,
+                           const int* tile_seq_len, const int* tile_q0, int num_tiles, int tile_rows, int T, int Hq, int Hkv,
                            int D, int causal, float scale, int* status, cudaStream_t stream) {
   if (num_tiles == 0 || T == 0) return 0;
   if (D != 64 && D != 128) return -2;
+  if (tile_rows != 128 && tile_rows != 256) return -3;
   static thread_local bool tl_context_bound = false;
   if (!tl_context_bound) {
     cudaFree(0);
@@ -350,7 +355,7 @@ extern "C" int sb_fmha_fwd(const void* qkv, void* out, float* lse, const int* ti
   CUtensorMap mq, mkv;
   int r = make_tensor_map_bf16_2d(&mq, qkv, width, T, width, 64, 128);
   if (r) return r;
-  r = make_tensor_map_bf16_2d(&mkv, qkv, width, T, width, 64, D == 128 ? 128 : 64);
+  r = make_tensor_map_bf16_2d(&mkv, qkv, width, T, width, 64, D == 128 && tile_rows == 256 ? 128 : 64);
   if (r) return r;
   FmhaFwdParams p;
   p.tile_seq_start = tile_seq_start; p.tile_seq_len = tile_seq_len; p.tile_q0 = tile_q0;
@@ -359,6 +364,9 @@ extern "C" int sb_fmha_fwd(const void* qkv, void* out, float* lse, const int* ti
   p.negate = scale < 0.f;
   p.scale_log2 = fmaxf(fabsf(scale) * 1.4426950408889634f, 1e-30f);  // 0 times a hidden score would not be a number
   p.status = status;
-  return D == 128 ? launch_fwd<128, 128, 1>(mq, mkv, p, num_tiles, stream)
-                  : launch_fwd<64, 64, 2>(mq, mkv, p, num_tiles, stream);
+  if (tile_rows == 128)
+    return D == 128 ? launch_fwd<128, 64, 1, 2>(mq, mkv, p, num_tiles, stream)
+                    : launch_fwd<64, 64, 1, 3>(mq, mkv, p, num_tiles, stream);
+  return D == 128 ? launch_fwd<128, 128, 2, 1>(mq, mkv, p, num_tiles, stream)
+                  : launch_fwd<64, 64, 2, 2>(mq, mkv, p, num_tiles, stream);
 }

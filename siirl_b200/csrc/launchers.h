@@ -101,7 +101,7 @@ int sb_ppo_token_loss(const float* logp, const float* old_logp, const float* adv
 extern "C" {
 // ---- fmha_fwd.cu / fmha_bwd.cu ----
 int sb_fmha_fwd(const void* qkv, void* out, float* lse, const int* tile_seq_start, const int* tile_seq_len,
-                const int* tile_q0, int num_tiles, int T, int Hq, int Hkv, int D, int causal, float scale,
+                const int* tile_q0, int num_tiles, int tile_rows, int T, int Hq, int Hkv, int D, int causal, float scale,
                 int* status, cudaStream_t stream);
 int sb_fmha_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,
                 float* dq_accum, float* dkv_accum, int* turn, void* dqkv, const int* tile_seq_start, const int* tile_seq_len,

@@ -15,7 +15,6 @@ from . import lib as _lib
 from . import reference as ref
 
 
-FWD_TILE = 256      # query rows of one block of the forward kernel
 _NUM_SMS = 148
 
 
@@ -50,15 +49,17 @@ class SeqInfo:
             self._pos = pos.to(self.device) if self.device is not None else pos
         return self._pos
 
-    def tiles(self, q_start: Optional[Sequence[int]] = None, rows: int = 128):
-        """(seq_start, seq_len, offset) int32 device tensors, one entry per tile of ``rows`` query rows; longest
-        sequences' last tiles first so the heaviest causal tiles start early.  ``q_start[i]`` leaves out the rows of sequence i below ``q_start[i] // 128 * 128``: chunked prefill
+    def tiles(self, hq: int, d: int, q_start: Optional[Sequence[int]] = None):
+        """(seq_start, seq_len, offset) int32 device tensors, one entry per tile of query rows, their number and the rows
+        of a tile for ``hq`` heads of width ``d``; longest sequences' last tiles first so the heaviest causal tiles start
+        early.  ``q_start[i]`` leaves out the rows of sequence i below ``q_start[i] // 128 * 128``: chunked prefill
         computes only the new rows."""
+        first = [int(q) // 128 * 128 for q in q_start] if q_start is not None else [0] * len(self.seqlens)
+        rows = fwd_tile_rows(len(first), self.total - sum(first), hq, d)
         if q_start is None and rows in self._tiles:
             return self._tiles[rows]
-        entries = [(self.cu_seqlens_cpu[i], n, t0) for i, n in enumerate(self.seqlens)
-                   for t0 in range(int(q_start[i]) // 128 * 128 if q_start is not None else 0, n, rows)]
-        tiles = self._device_tiles(sorted(entries, key=lambda e: -e[2]))
+        entries = [(self.cu_seqlens_cpu[i], n, t0) for i, n in enumerate(self.seqlens) for t0 in range(first[i], n, rows)]
+        tiles = self._device_tiles(sorted(entries, key=lambda e: -e[2])) + (rows,)
         if q_start is None:
             self._tiles[rows] = tiles
         return tiles
@@ -74,6 +75,19 @@ class SeqInfo:
     def _device_tiles(self, entries):
         mk = lambda k: torch.tensor([e[k] for e in entries], dtype=torch.int32, device=self.device)  # noqa: E731
         return (mk(0), mk(1), mk(2), len(entries))
+
+
+def fwd_tile_rows(sequences: int, query_rows: int, hq: int, d: int) -> int:
+    """Query rows of one block of the forward kernel: 256, or 128 where a second tile of 128 would mostly stand idle.  A block
+    of 128 rows takes half an SM (d = 128) or a third, so short sequences hide each other's latencies; a longer one fetches
+    its keys twice as often.  256 / 128 rows, us, causal: d = 128, 28 / 4 heads: 256 x 64 tokens 301 / 128, 128 x 128:
+    188 / 119, 64 x 200: 149 / 123, 40 x 384: 192 / 147, 32 x 512: 192 / 176 but 216 / 237 not causal, and 4 x 384 with
+    16 heads, one block an SM, 12 / 14; d = 64, 14 / 2: 256 x 64: 50 / 37, 128 x 128: 43 / 35, 64 x 160 30 / 31."""
+    if query_rows <= 128 * sequences:
+        return 128
+    if d == 128 and query_rows <= 384 * sequences and -(-query_rows // 256) * hq > _NUM_SMS:
+        return 128
+    return 256
 
 
 def bwd_head_splits(seqlens: Sequence[int], hq: int, hkv: int, causal: bool) -> int:
@@ -126,9 +140,9 @@ class _AttnFn(torch.autograd.Function):
         T = qkv.shape[0]
         out = torch.empty(T, hq * d, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-        ts, tl, t0, n = info.tiles(q_start, FWD_TILE)
-        rc = L.sb_fmha_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T,
-                           hq, hkv, d, int(causal), ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)),
+        ts, tl, t0, n, rows = info.tiles(hq, d, q_start)
+        rc = L.sb_fmha_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, rows,
+                           T, hq, hkv, d, int(causal), ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)),
                            _lib.stream())
         _lib.check(rc, "sb_fmha_fwd")
         ctx.save_for_backward(qkv, out, lse)

@@ -30,7 +30,7 @@ import torch
 import torch.distributed as dist
 
 from ..ops import lib as _lib
-from ..ops.attention import FWD_TILE, SeqInfo, fmha_bwd
+from ..ops.attention import SeqInfo, fmha_bwd
 from .ulysses import _PullBlock
 
 
@@ -65,8 +65,8 @@ def _block_fwd(qkv, info: SeqInfo, hq, hkv, d, causal, scale) -> Tuple[torch.Ten
     L = _lib.get_lib()
     out = torch.empty(T, hq * d, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-    ts, tl, t0, n = info.tiles(rows=FWD_TILE)
-    _lib.check(L.sb_fmha_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n,
+    ts, tl, t0, n, rows = info.tiles(hq, d)
+    _lib.check(L.sb_fmha_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, rows,
                              T, hq, hkv, d, int(causal), ctypes.c_float(scale),
                              _lib.ptr(_lib.status_word(qkv.device)), _lib.stream()), "sb_fmha_fwd")
     return out, lse

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from siirl_b200.ops import lib, reference as ref
-from siirl_b200.ops.attention import SeqInfo, attention_packed, bwd_head_splits, bwd_ordered
+from siirl_b200.ops.attention import SeqInfo, attention_packed, bwd_head_splits, bwd_ordered, fwd_tile_rows
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -74,6 +74,28 @@ def test_attention_fwd_tiles(d, hq, hkv, scale, gain, causal):
     T = sum(seqlens)
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
     qkv = (gain * torch.randn(T, (hq + 2 * hkv) * d, device=DEV)).to(torch.bfloat16)
+    out = attention_packed(qkv, SeqInfo(seqlens, device=DEV), hq, hkv, d, causal=causal, scale=scale)
+    lib.check_status()
+    q, k, v = qkv.float().split([hq * d, hkv * d, hkv * d], dim=-1)
+    want = ref.attention_varlen(q.reshape(T, hq, d), k.reshape(T, hkv, d), v.reshape(T, hkv, d),
+                                torch.tensor([0] + list(torch.tensor(seqlens).cumsum(0))), causal=causal,
+                                scale=scale).reshape(T, hq * d)
+    # weights and outputs are rounded to bf16 (2^-9 each, relative): 1e-2 of a row leaves a factor of two and a half
+    row_err = (out.float() - want).norm(dim=1) / want.norm(dim=1)
+    assert row_err.max().item() < 1e-2, row_err.argmax().item()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("d,hq,hkv,seqlens,scale", [(128, 4, 2, [1, 127, 128, 64, 65, 63, 129, 2], None),
+                                                    (64, 7, 1, [1, 127, 128, 64, 65, 63, 129, 2], -0.2),
+                                                    (128, 4, 1, [129, 385, 256, 257, 512] * 12, None), (64, 2, 2, [20] * 40 + [1500], 0.0)])
+def test_attention_fwd_short_sequences(d, hq, hkv, seqlens, scale, causal):
+    """The form with one query tile of 128 rows: sequences around its tiles and more key tiles than the ring has stages."""
+    torch.manual_seed(1)
+    T = sum(seqlens)
+    assert fwd_tile_rows(len(seqlens), T, hq, d) == 128
+    scale = scale if scale is not None else 1.0 / math.sqrt(d)
+    qkv = (0.7 * torch.randn(T, (hq + 2 * hkv) * d, device=DEV)).to(torch.bfloat16)
     out = attention_packed(qkv, SeqInfo(seqlens, device=DEV), hq, hkv, d, causal=causal, scale=scale)
     lib.check_status()
     q, k, v = qkv.float().split([hq * d, hkv * d, hkv * d], dim=-1)

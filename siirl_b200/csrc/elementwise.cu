@@ -46,35 +46,48 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // RMSNorm forward:  h = x (+ residual);  y = h * rsqrt(mean(h^2) + eps) * w
 // x may also be the fp32 partial sums of a split contraction (`slabs`), added up here: a pass of their own over so few
 // rows costs a launch (2.9 us against some 0.3 us of memory time for 8 x 896) and a rounding.
+// Bound by memory.  All of a row's loads come before its first store, and the weights before the rows: the compiler may not
+// move them across a store by itself (9600 x 3584: 66 us with the stores of the sum in between, 46 us so).  Rows of up to
+// 2048 columns: eight blocks on an SM, as many as the grid has (9600 x 1024 with six: 17.7 us, with eight 14.7).
 // ---------------------------------------------------------------------------------------
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxChunks = 4;  // hidden <= 256 * 8 * 4 = 8192
 
-template <int CH>
-__global__ void __launch_bounds__(kNormThreads)
+template <int CH, bool SLABS>
+__global__ void __launch_bounds__(kNormThreads, CH == 1 ? 8 : CH == 2 ? 4 : 2)
 rmsnorm_fwd_kernel(const __nv_bfloat16* x, const float* slabs, long long slab_stride, int splits,
                    const __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* h_out,
                    float* rstd_out, int T, int H, float eps) {
   __shared__ float red[32];
   chain_sync();
   const int nvec = H / 8;
+  uint4 w4[CH];
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int vi = threadIdx.x + c * kNormThreads;
+    if (vi < nvec) w4[c] = reinterpret_cast<const uint4*>(w)[vi];
+  }
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     float hv[CH][8];
+    uint4 x4[CH], r4[CH];
     float ss = 0.f;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       const int vi = threadIdx.x + c * kNormThreads;
       if (vi < nvec) {
-        if (slabs) {
-          slab_sum8(slabs + (size_t)row * H + vi * 8, slab_stride, splits, hv[c]);
-        } else {
-          uint4 xv = reinterpret_cast<const uint4*>(x + (size_t)row * H)[vi];
-          bf16x8_to_float(xv, hv[c]);
-        }
+        if (SLABS) slab_sum8(slabs + (size_t)row * H + vi * 8, slab_stride, splits, hv[c]);
+        else x4[c] = reinterpret_cast<const uint4*>(x + (size_t)row * H)[vi];
+        if (residual) r4[c] = reinterpret_cast<const uint4*>(residual + (size_t)row * H)[vi];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int vi = threadIdx.x + c * kNormThreads;
+      if (vi < nvec) {
+        if (!SLABS) bf16x8_to_float(x4[c], hv[c]);
         if (residual) {
           float rv[8];
-          uint4 r4 = reinterpret_cast<const uint4*>(residual + (size_t)row * H)[vi];
-          bf16x8_to_float(r4, rv);
+          bf16x8_to_float(r4[c], rv);
 #pragma unroll
           for (int i = 0; i < 8; ++i) hv[c][i] += rv[i];
           if (h_out) {
@@ -96,7 +109,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* x, const float* slabs, long long slab_st
       const int vi = threadIdx.x + c * kNormThreads;
       if (vi < nvec) {
         float wv[8], o[8];
-        bf16x8_to_float(reinterpret_cast<const uint4*>(w)[vi], wv);
+        bf16x8_to_float(w4[c], wv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = hv[c][i] * rstd * wv[i];
         reinterpret_cast<uint4*>(y + (size_t)row * H)[vi] = float_to_bf16x8(o);
@@ -472,7 +485,7 @@ static int rmsnorm_fwd(const void* x, const float* slabs, long long slab_stride,
   const int ch = (H / 8 + kNormThreads - 1) / kNormThreads;
   const int grid = T < num_sms() * 8 ? T : num_sms() * 8;
 #define SB_LAUNCH(CH)                                                                                     \
-  return launch_chained(rmsnorm_fwd_kernel<CH>, grid, kNormThreads, 0, stream,                            \
+  return launch_chained(slabs ? rmsnorm_fwd_kernel<CH, true> : rmsnorm_fwd_kernel<CH, false>, grid, kNormThreads, 0, stream, \
       (const __nv_bfloat16*)x, slabs, slab_stride, splits, (const __nv_bfloat16*)residual,                  \
       (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, T, H, eps)
   switch (ch) {

@@ -320,3 +320,18 @@ def test_rmsnorm_backward_widths(T, H):
     # one rounding to bf16 (2^-9 relative); the weight's gradient is rounded after a 32-bit sum
     assert ((x.grad.double() - want).norm() / want.norm()).item() < 3e-3 and torch.equal(x.grad, r.grad)
     assert ((w.grad.double() - wd.grad).norm() / wd.grad.norm()).item() < 4e-3
+
+
+@pytest.mark.parametrize("with_residual", [True, False])
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 2048), (2500, 2056), (1300, 3584), (5, 4104), (1200, 8192)])
+def test_rmsnorm_forward_widths(T, H, with_residual):
+    """Every number of vectors per thread, at its edges, with fewer rows than blocks and more."""
+    torch.manual_seed(0)
+    x, r = (torch.randn(T, H, device=DEV).to(torch.bfloat16) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, device=DEV)).to(torch.bfloat16)
+    y, h = ops.rmsnorm(x, w, 1e-6, residual=r if with_residual else None)
+    if with_residual:
+        assert torch.equal(h, (x.float() + r.float()).to(torch.bfloat16))
+    want = h.double() * torch.rsqrt(h.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    # one rounding to bf16 (2^-9 relative) of a value that 32 bits give to 1e-6
+    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()

@@ -335,3 +335,9 @@ def test_rmsnorm_forward_widths(T, H, with_residual):
     want = h.double() * torch.rsqrt(h.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
     # one rounding to bf16 (2^-9 relative) of a value that 32 bits give to 1e-6
     assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("T,I", [(9000, 8), (15000, 1048), (7, 768), (2000, 264), (40, 520)])
+def test_swiglu_narrow_rows(T, I):
+    """Rows that share a block, rows divided evenly over blocks, and single rows or pairs per thread."""
+    test_swiglu_rows(T, I)

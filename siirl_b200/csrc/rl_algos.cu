@@ -96,8 +96,9 @@ __global__ void row_sum_kernel(const float* x, float* out, int B, int R) {
 }
 
 // Up to kGroupScanRows rows: every block finds its row's group among all rows' scores by itself, twice the scan of a few
-// KB out of L2 for two launches instead of a fill and four (15 us of launches and gaps for 256 rows).  Above that the scans
-// (rows x rows) would cost more than they save.
+// KB out of L2 for two launches instead of a fill and four (15 us of launches and gaps for 256 rows).  The work is rows x
+// rows x blocks of a row, of which the caller takes one from num_sms * 8 rows on.  us, the four launches and this:
+// 256 x 4096 14.4, 7.6; 1024 x 4096 23.3, 11.3; 2048 x 4096 46.8, 32.7; 2048 x 8192 75.8, 63.1.
 constexpr int kGroupScanRows = 2048;
 
 __global__ void __launch_bounds__(256) grpo_scan_kernel(const float* scores, const int* gid, const float* mask, float* adv,
@@ -385,9 +386,12 @@ extern "C" int sb_grpo_group_adv(const float* rewards, const float* mask, const 
   if (B == 0 || R == 0) return 0;
   const dim3 grid((R + 255) / 256 > 8 ? 8 : (R + 255) / 256, B);
   if (B <= kGroupScanRows) {
+    // every block of a row scans all rows: no more blocks than the SMs hold at once, each with more columns
+    const int fit = num_sms() * 8 / B > 1 ? num_sms() * 8 / B : 1;
+    const dim3 scan_grid((int)grid.x < fit ? grid.x : fit, B);
     const int rc = launch_chained(row_sum_kernel, (B * 32 + 127) / 128, 128, 0, stream, rewards, scores_ws, B, R);
     if (rc) return rc;
-    return launch_chained(grpo_scan_kernel, grid, 256, 0, stream, (const float*)scores_ws, gid, mask, adv, B, R, G, eps,
+    return launch_chained(grpo_scan_kernel, scan_grid, 256, 0, stream, (const float*)scores_ws, gid, mask, adv, B, R, G, eps,
                           norm_by_std);
   }
   const cudaError_t me = cudaMemsetAsync(group_ws, 0, sizeof(float) * 3 * G, stream);

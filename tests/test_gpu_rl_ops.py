@@ -113,3 +113,9 @@ def test_fused_ppo_loss_matches_torch(mode, agg):
     torch.testing.assert_close(met["ppo_kl"], ppo_kl.detach(), rtol=1e-4, atol=1e-5)
     torch.testing.assert_close(logp.grad, lp2.grad, rtol=1e-3, atol=1e-6)
     torch.testing.assert_close(ent.grad, ent2.grad, rtol=1e-4, atol=1e-7)
+
+
+@pytest.mark.parametrize("B,R,G", [(2048, 3000, 300), (700, 2100, 90), (1185, 257, 1185)])
+def test_grpo_group_adv_many_rows(B, R, G):
+    """One block per row, each with many columns, and two."""
+    test_grpo_group_adv_sizes(B, R, G)

@@ -91,18 +91,23 @@ def fwd_tile_rows(sequences: int, query_rows: int, hq: int, d: int) -> int:
 
 
 def bwd_head_splits(seqlens: Sequence[int], hq: int, hkv: int, causal: bool) -> int:
-    """Blocks over which the backward kernel divides the q heads of a kv head.  Splitting adds fp32 sums of dK and dV and a
-    pass that converts them, so it is done only as far as the block with most steps would outlast an SM's average share:
-    (28 / 4 heads, 8 x 2048: share 0.54, whole 0.86 ms, halves 1.05; 14 / 2 heads, 1 x 9900: share 1.9, whole 1.21 ms,
-    thirds 0.72)."""
+    """Blocks over which the backward kernel divides the q heads of a kv head: more of them shorten the longest block, but
+    each costs some five steps of its own (loading K and V, writing dK and dV), and another where a share's dK and dV go
+    through a buffer.  In steps of one 128 x 128 tile of one head the pass takes the longest block, or the SMs' average and
+    a tail that shrinks with the blocks an SM gets.  Forward and backward, us, for 1, 2, 3, 4, 7 blocks, causal: 28 / 4
+    heads, d = 128: 32 x 64: 90, 108, 116, 126, 157; 16 x 128: 79, 75, 89, 88, 113; 4 x 512: 150, 116, 108, 113, 126;
+    1 x 1024: 231, 154, 128, 103, 93; 4 x 2048: 841, 720, 738, 762, 836; 14 / 2 heads, d = 64: 1 x 9000: 1300, 874, 846,
+    825, 845; 16 x 1000: 326, 301, 311, 326, 371."""
     rep = hq // hkv
     tiles = [(n + 127) // 128 for n in seqlens]
-    total = sum(t * (t + 1) // 2 if causal else t * t for t in tiles) * hq
-    longest = max(tiles, default=0)
-    for splits in range(1, rep):
-        if -(-rep // splits) * longest * _NUM_SMS <= total:
-            return splits
-    return rep
+    average = sum(t * (t + 1) // 2 if causal else t * t for t in tiles) * hq / _NUM_SMS
+    longest, blocks = max(tiles, default=0), sum(tiles) * hkv
+
+    def steps(splits):
+        block, per_sm = -(-rep // splits) * longest, blocks * splits / _NUM_SMS
+        own = 5 * math.ceil(per_sm) + (per_sm if splits > 1 else 0)
+        return max(block, average + block / max(1.0, per_sm) ** 2) + own
+    return min(range(1, rep + 1), key=steps)
 
 
 def bwd_ordered(max_seqlen: int, d: int, causal: bool) -> bool:

@@ -323,3 +323,11 @@ def test_tracking_backends(tmp_path, monkeypatch, capsys):
     assert "params" in kinds and ("metrics" in kinds) and kinds[-1] == "end"
     logged = next(c for c in calls if c[0] == "metrics")
     assert logged[2] == 3 and logged[1] == {"x/y_at_4": 1.5} and ("run", "7", "exp") in calls
+
+
+def test_attention_backward_head_splits():
+    """Few blocks are divided, blocks that fill the SMs and short ones are not."""
+    from siirl_b200.ops.attention import bwd_head_splits
+    assert bwd_head_splits([1024], 28, 4, True) == 7 and bwd_head_splits([9900], 14, 2, True) > 1
+    assert all(bwd_head_splits([n] * k, 28, 4, c) == 1 for n, k in ((64, 32), (128, 32), (1000, 16)) for c in (True, False))
+    assert bwd_head_splits([4096] * 4, 8, 8, True) == 1 and bwd_head_splits([], 4, 2, True) == 1

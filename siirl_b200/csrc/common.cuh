@@ -460,7 +460,9 @@ inline int launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, siz
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // the caller gets it; the next launch of anyone must not find it again
+  return (int)e;
 }
 
 // ---------------------------------------------------------------------------------------

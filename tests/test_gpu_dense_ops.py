@@ -341,3 +341,15 @@ def test_rmsnorm_forward_widths(T, H, with_residual):
 def test_swiglu_narrow_rows(T, I):
     """Rows that share a block, rows divided evenly over blocks, and single rows or pairs per thread."""
     test_swiglu_rows(T, I)
+
+
+def test_refused_launch_leaves_no_error_behind():
+    """A launch that the runtime refuses (a grid of 70000 in y) is reported by its own call and by none after it."""
+    import ctypes
+    logits = torch.zeros(1, 128, device=DEV)
+    tok, lp, ws = torch.zeros(1, dtype=torch.int64, device=DEV), torch.zeros(1, device=DEV), torch.zeros(4, device=DEV)
+    rc = lib.get_lib().sb_sample(lib.ptr(logits), lib.ptr(logits), ctypes.c_longlong(128), ctypes.c_float(1.0),
+                                 ctypes.c_ulonglong(0), ctypes.c_ulonglong(0), None, lib.ptr(tok), lib.ptr(lp), 1, 128,
+                                 lib.ptr(ws), 70000, lib.stream())
+    assert rc != 0
+    assert float((lp + 1).sum()) == 1.0

@@ -140,13 +140,16 @@ __device__ __forceinline__ float2 add_mul2(float2 a, float2 b, float2 f) {  // (
 }
 
 // 16 warps: 0-7 P and dS (thread = kv row and one half of the query columns), 8-11 dQ, 12 TMA, 13 MMA issuer, 14 row
-// statistics.  The launch's 128 registers a thread are shared out as 144, 144, 152 and 72 to the four warpgroups.
-constexpr int kBwdThreads = 512;
+// statistics.  The launch's 128 registers a thread are shared out as 144, 144, 152 and 72 to the four warpgroups.  __maxnreg__
+// and not __launch_bounds__: it is the directive from which setmaxnreg takes the count at launch, while launch bounds only
+// limit what the compiler may use.
+constexpr int kBwdThreads = 512, kBwdRegs = 128;
 constexpr int kRegsMath = 144, kRegsDq = 152, kRegsIssue = 72;
-static_assert(2 * kRegsMath + kRegsDq + kRegsIssue <= 4 * 128, "more registers than the launch has");
+static_assert(2 * kRegsMath + kRegsDq + kRegsIssue <= 4 * kBwdRegs, "more registers than the launch has");
+static_assert(kBwdThreads * kBwdRegs <= 65536, "more registers than an SM has");
 
 template <int D, bool ORDERED>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __maxnreg__(kBwdRegs)
 fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_do,
                 FmhaBwdParams p) {
   using L = BwdSmem<D>;
@@ -617,7 +620,7 @@ static int launch_bwd(const CUtensorMap& mqkv, const CUtensorMap& mdo, const Fmh
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
     if (e != cudaSuccess) return (int)e;
-    // the warpgroups' shares are drawn from the registers that the block is launched with
+    // the warpgroups' shares are drawn from the registers that the block is launched with: with fewer they would wait for good
     if (attr.numRegs * 4 < 2 * kRegsMath + kRegsDq + kRegsIssue) return -6;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
     if (e != cudaSuccess) return (int)e;

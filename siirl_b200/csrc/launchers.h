@@ -90,6 +90,7 @@ extern "C" {
 // ---- rl_algos.cu ----
 int sb_gae_scan(const float* rewards, const float* values, const float* mask, float* adv, float* ret, int B,
                 int R, float gamma, float lam, cudaStream_t stream);
+int sb_grpo_scan_rows();
 int sb_grpo_group_adv(const float* rewards, const float* mask, const int* gid, float* scores_ws, float* group_ws,
                       float* adv, int B, int R, int G, float eps, int norm_by_std, cudaStream_t stream);
 int sb_ppo_token_loss(const float* logp, const float* old_logp, const float* adv, const float* mask,

@@ -380,6 +380,9 @@ extern "C" int sb_gae_scan(const float* rewards, const float* values, const floa
   return (int)cudaGetLastError();
 }
 
+// rows up to which sb_grpo_group_adv launches two kernels (else four)
+extern "C" int sb_grpo_scan_rows() { return kGroupScanRows; }
+
 extern "C" int sb_grpo_group_adv(const float* rewards, const float* mask, const int* gid, float* scores_ws,
                                  float* group_ws, float* adv, int B, int R, int G, float eps, int norm_by_std,
                                  cudaStream_t stream) {

@@ -135,6 +135,7 @@ def fmha_bwd(qkv, out, lse, dout, info: SeqInfo, hq: int, hkv: int, d: int, caus
                        _lib.ptr(dkv_acc), _lib.ptr(turn), _lib.ptr(dqkv), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T,
                        hq, hkv, d, int(causal), splits, ctypes.c_float(scale), _lib.ptr(_lib.status_word(qkv.device)), _lib.stream())
     _lib.check(rc, "sb_fmha_bwd")
+    _lib.add_launches(int(splits > 1))
     return dqkv
 
 

@@ -407,7 +407,8 @@ def _rope_native(qkv: torch.Tensor, n_heads_rot: int, head_dim: int, positions: 
     args = (_lib.ptr(pos), _lib.ptr(cos_tab), _lib.ptr(sin_tab), T, qkv.stride(0), n_heads_rot, head_dim, rows, s0, s1,
             ctypes.c_float(sign), _lib.stream())
     rc = L.sb_rope_rows(_lib.ptr(qkv), _lib.ptr(out), *args)
-    if rc == -2:        # odd widths
+    if rc == -2:        # odd widths; nothing was launched
+        _lib.add_launches(-1)
         out.copy_(qkv)
         rc = L.sb_rope(_lib.ptr(out), *args)
     _lib.check(rc, "sb_rope")

@@ -135,6 +135,7 @@ def decode_attention(q_rows: torch.Tensor, cache_layer: torch.Tensor, seq_lens: 
                                               _lib.ptr(ws_o), _lib.ptr(ws_lse), B, n_heads, n_kv_heads, head_dim,
                                               ctypes.c_float(scale), _lib.ptr(_lib.status_word(q_rows.device)),
                                               _lib.stream()), "sb_fmha_decode_split")
+            _lib.add_launches(int(ws_lse.numel() > B * n_heads))    # several chunks are merged
             return out
         _lib.check(L.sb_fmha_decode(_lib.ptr(q_rows), q_rows.stride(0), _lib.ptr(cache_layer),
                                     ctypes.c_longlong(cache_layer.shape[0]), _lib.ptr(seq_lens), _lib.ptr(block_table),

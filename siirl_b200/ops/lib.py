@@ -18,10 +18,12 @@ _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libsiirl_b200.so"
 _lib: Optional["_CountingLib"] = None
 _status_words: dict[int, torch.Tensor] = {}
 
-# kernels launched by one call of each entry point (for the launch counter of the benchmark)
-_KERNELS_PER_CALL = {"sb_rmsnorm_bwd": 2, "sb_grpo_group_adv": 2, "sb_ppo_token_loss": 2, "sb_fmha_bwd": 3,
-                     "sb_kk_partition": 0, "sb_rmsnorm_bwd_blocks": 0, "sb_colsum_blocks": 0, "sb_colsum_bf16": 2, "sb_gemm_set_pair_kernel": 0,
-                     "sb_recurrence_prefill": 2, "sb_attn_window_decode": 2, "sb_latent_decode": 2,
+# kernels launched by one call of each entry point (for the launch counter of the benchmark); callers add what depends on
+# the sizes
+_KERNELS_PER_CALL = {"sb_rmsnorm_bwd": 2, "sb_grpo_group_adv": 2, "sb_grpo_scan_rows": 0, "sb_ppo_token_loss": 2,
+                     "sb_fmha_bwd": 3, "sb_kk_partition": 0, "sb_rmsnorm_bwd_blocks": 0, "sb_colsum_blocks": 0,
+                     "sb_colsum_bf16": 2, "sb_gemm_set_pair_kernel": 0, "sb_fmha_decode_chunk_tiles": 0,
+                     "sb_attn_window_decode_chunks": 0, "sb_recurrence_prefill": 2, "sb_attn_window_decode": 2, "sb_latent_decode": 2,
                      "sb_delta_prefill": 3}
 
 

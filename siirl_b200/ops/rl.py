@@ -57,6 +57,7 @@ def grpo_group_advantage(rewards: torch.Tensor, mask: torch.Tensor, group_ids: t
     _lib.check(L.sb_grpo_group_adv(_lib.ptr(r), _lib.ptr(m), _lib.ptr(gid), _lib.ptr(scores), _lib.ptr(ws),
                                    _lib.ptr(adv), B, R, num_groups, _f(eps), int(norm_by_std), _lib.stream()),
                "sb_grpo_group_adv")
+    _lib.add_launches(2 if B > L.sb_grpo_scan_rows() else 0)
     return adv
 
 

@@ -47,4 +47,5 @@ def sample(logits: torch.Tensor, temperature: float = 1.0, top_k: int = -1, top_
                            ctypes.c_float(temperature), ctypes.c_ulonglong(seed & (2 ** 64 - 1)),
                            ctypes.c_ulonglong(step), _lib.ptr(step_dev), _lib.ptr(tokens), _lib.ptr(logp), B, V,
                            _lib.ptr(ws), splits, _lib.stream()), "sb_sample")
+    _lib.add_launches(int(splits > 1))
     return tokens, logp

@@ -353,3 +353,33 @@ def test_refused_launch_leaves_no_error_behind():
                                  lib.ptr(ws), 70000, lib.stream())
     assert rc != 0
     assert float((lp + 1).sum()) == 1.0
+
+
+def test_launch_counter_follows_the_sizes():
+    """Calls whose number of kernels depends on the sizes."""
+    from siirl_b200.ops import kv_cache as kvc, rl
+    from siirl_b200.ops.attention import SeqInfo, attention_packed, bwd_head_splits
+    from siirl_b200.ops.sampling import sample
+
+    def launches(fn):
+        before = lib.launch_count()
+        fn()
+        return lib.launch_count() - before
+    for rows, want in ((8, 2), (2048, 2), (2049, 4)):
+        x, gid = torch.ones(rows, 3, device=DEV), torch.zeros(rows, dtype=torch.int32, device=DEV)
+        assert launches(lambda: rl.grpo_group_advantage(x, x, gid, 1)) == want
+    for seqlens, hq, want in (([256], 2, 4), ([64] * 300, 2, 3), ([256], 1, 3)):
+        assert (bwd_head_splits(seqlens, hq, 1, True) > 1) == (want == 4)
+        x = torch.randn(sum(seqlens), (hq + 2) * 64, device=DEV).to(torch.bfloat16).requires_grad_()
+        out = attention_packed(x, SeqInfo(seqlens, device=DEV), hq, 1, 64)
+        assert launches(lambda: out.backward(torch.ones_like(out))) == want
+    q, table = torch.zeros(2, 6 * 64, device=DEV, dtype=torch.bfloat16), torch.arange(34, dtype=torch.int32, device=DEV).reshape(2, 17)
+    cache, n = torch.zeros(34, 2, 1, 64, 64, device=DEV, dtype=torch.bfloat16), torch.ones(2, dtype=torch.int32, device=DEV)
+    for blocks, want in ((16, 1), (17, 2)):
+        t = table[:, :blocks].contiguous()
+        assert launches(lambda: kvc.decode_attention(q, cache, n, t, 4, 1, 64)) == want
+    for V, want in ((4000, 1), (40000, 2)):
+        assert launches(lambda: sample(torch.zeros(2, V, device=DEV))) == want
+    cos, sin = ops.rope_tables(24, 8, 10000.0, device=DEV)
+    x = torch.zeros(4, 5 * 24, device=DEV, dtype=torch.bfloat16)
+    assert launches(lambda: ops.rope(x, 3, 24, torch.arange(4, device=DEV), cos, sin, None)) == 1

@@ -76,7 +76,8 @@ def set_pair_kernel(enabled: bool) -> bool:
 def _column_sums(x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 column sums of ``x [T, N]``, added to ``out`` when it is given."""
     T, N = x.shape
-    if x.dtype != torch.bfloat16 or N % 8 or x.data_ptr() % 16 or (out is not None and not out.is_contiguous()):
+    if x.dtype != torch.bfloat16 or N % 8 or x.data_ptr() % 16 or not x.is_contiguous() or (
+            out is not None and (not out.is_contiguous() or out.dtype != torch.float32)):
         s = x.float().sum(0)
         return s if out is None else out.add_(s)
     L = _lib.get_lib()

@@ -383,3 +383,19 @@ def test_launch_counter_follows_the_sizes():
     cos, sin = ops.rope_tables(24, 8, 10000.0, device=DEV)
     x = torch.zeros(4, 5 * 24, device=DEV, dtype=torch.bfloat16)
     assert launches(lambda: ops.rope(x, 3, 24, torch.arange(4, device=DEV), cos, sin, None)) == 1
+
+
+def test_column_sums_of_other_layouts():
+    """Rows apart and sums kept in another type go through the plain form."""
+    torch.manual_seed(0)
+    x = torch.randn(300, 64, device=DEV).to(torch.bfloat16)
+    want = x.double().sum(0)
+    for src, out, tol in ((x, torch.zeros(64, device=DEV, dtype=torch.bfloat16), 2 ** -8),
+                          (x, torch.zeros(64, device=DEV, dtype=torch.float64), 1e-5),
+                          (torch.cat([x, x], 1)[:, :64], torch.zeros(64, device=DEV), 1e-5),
+                          (torch.cat([x, x], 1)[:, :64], None, 1e-5),
+                          (x, torch.zeros(64, 2, device=DEV)[:, 0], 1e-5)):
+        got = dense._column_sums(src, out)
+        assert out is None or got.data_ptr() == out.data_ptr() and got.dtype == out.dtype
+        # one rounding to the output's type of a 32-bit sum of 300 numbers
+        assert ((got.double() - want).abs() <= tol * (want.abs() + 20)).all()

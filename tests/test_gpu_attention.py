@@ -68,7 +68,7 @@ def test_attention_fwd_bwd(cfg, causal):
                                                  (64, 2, 1, 0.0, 0.5), (128, 2, 1, None, 4.0), (64, 2, 2, None, 4.0)])
 def test_attention_fwd_tiles(d, hq, hkv, scale, gain, causal):
     """Sequences around the tile sizes (128 keys, 256 rows), more key tiles than the ring has stages, scales of either
-    sign, and scores so far apart that the running maximum moves by more than the lazy bound."""
+    sign, and scores so far apart that the running maximum moves and the output so far is scaled."""
     seqlens = [1, 127, 128, 129, 255, 256, 257, 385, 1500, 2]
     torch.manual_seed(1)
     T = sum(seqlens)

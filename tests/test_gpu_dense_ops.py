@@ -219,17 +219,16 @@ def test_partial_sums_and_their_consumers(rows, hidden, inter, hq, hkv, d):
     h, w = torch.randn_like(x), (1 + 0.1 * torch.randn(hidden, device=DEV)).to(torch.bfloat16)
     wo, wg, wq, bias = mk(hidden, hidden), mk(2 * inter, hidden), mk((hq + 2 * hkv) * d, hidden), mk((hq + 2 * hkv) * d)
     so, sg, sq = (ops.linear_slabs(x, t) for t in (wo, wg, wq))
-    assert so is not None and sq is not None
+    assert so is not None and sq is not None and sg is not None
     y, hs = ops.rmsnorm_slabs(so, w, 1e-6, h)
     want = x.double() @ wo.double().T + h.double()
     # results rounded to bf16 once (2^-9 relative), the norm's input as well
     assert ((hs.double() - want).norm() / want.norm()).item() < 3e-3
     want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double()
     assert ((y.double() - want).norm() / want.norm()).item() < 5e-3
-    if sg is not None:
-        g, u = (x.double() @ wg.double().T).chunk(2, -1)
-        want = torch.nn.functional.silu(g) * u
-        assert ((ops.swiglu_slabs(sg).double() - want).norm() / want.norm()).item() < 3e-3
+    g, u = (x.double() @ wg.double().T).chunk(2, -1)
+    want = torch.nn.functional.silu(g) * u
+    assert ((ops.swiglu_slabs(sg).double() - want).norm() / want.norm()).item() < 3e-3
     cos, sin = ops.rope_tables(d, 64, 10000.0, device=DEV)
     pos = (torch.arange(rows, device=DEV) % 64).to(torch.int32)
     seq = torch.arange(rows, device=DEV, dtype=torch.int32)
@@ -399,3 +398,35 @@ def test_column_sums_of_other_layouts():
         assert out is None or got.data_ptr() == out.data_ptr() and got.dtype == out.dtype
         # one rounding to the output's type of a 32-bit sum of 300 numbers
         assert ((got.double() - want).abs() <= tol * (want.abs() + 20)).all()
+
+
+@pytest.mark.parametrize("clip", [0.0, 0.5])
+@pytest.mark.parametrize("n,shift", [(1, 0), (3, 0), (4, 0), (5, 0), (1027, 0), (1030, 1), (64 * 148 * 1024 + 261, 0),
+                                     (64 * 148 * 1024 * 2 + 12, 0), (300001, 3)])
+def test_adamw_kernel(n, shift, clip):
+    """Every element is updated once and none beyond the last: vectors and the rest, pieces of one and of several sweeps,
+    blocks without work, and buffers that do not start on 16 bytes."""
+    import ctypes
+    torch.manual_seed(0)
+    guard = 8
+    mk = lambda dtype=torch.float32: torch.randn(shift + n + guard, device=DEV).to(dtype)  # noqa: E731
+    w, m, v, g, p = mk(), mk(), mk().abs(), mk(), mk(torch.bfloat16)
+    sumsq, norm = (torch.zeros(1, device=DEV) for _ in range(2))
+    f, at = ctypes.c_float, lambda t: ctypes.c_void_p(t.data_ptr() + shift * t.element_size())
+    before = [t.clone() for t in (w, m, v, p)]
+    inside = slice(shift, shift + n)
+    sumsq += g[inside].double().square().sum().float()
+    lr, b1, b2, eps, wd, step, scale = 1e-2, 0.9, 0.99, 1e-8, 0.1, 3, 0.25
+    lib.check(lib.get_lib().sb_adamw_step(at(w), at(m), at(v), at(g), at(p), lib.ptr(sumsq), lib.ptr(norm), ctypes.c_longlong(n),
+                                          f(lr), f(b1), f(b2), f(eps), f(wd), step, f(clip), f(scale), lib.stream()), "adamw")
+    total = sumsq.double().sqrt() * scale
+    assert abs(float(norm) / float(total) - 1) < 1e-5
+    g64 = g[inside].double() * scale * (min(1.0, clip / (float(total) + 1e-6)) if clip else 1.0)
+    m64 = b1 * before[1][inside].double() + (1 - b1) * g64
+    v64 = b2 * before[2][inside].double() + (1 - b2) * g64 * g64
+    w64 = before[0][inside].double() * (1 - lr * wd) - lr * (m64 / (1 - b1 ** step)) / ((v64 / (1 - b2 ** step)).sqrt() + eps)
+    # a handful of 32-bit operations each; one rounding to bf16 of the weight
+    for got, want, tol in ((m, m64, 1e-6), (v, v64, 1e-6), (w, w64, 1e-5), (p, w64, 2 ** -8)):
+        assert ((got[inside].double() - want).abs() <= tol * want.abs() + 1e-6).all()
+    for got, old in zip((w, m, v, p), before):
+        assert torch.equal(got[:shift], old[:shift]) and torch.equal(got[shift + n:], old[shift + n:])

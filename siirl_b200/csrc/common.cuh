@@ -487,6 +487,20 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return y;
 }
 
+// two at a time
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(d)
+      : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
+  return *reinterpret_cast<float2*>(&d);
+}
+
 // v = sum over `splits` slabs of the eight floats at p (16-byte aligned), slab_stride floats apart
 __device__ __forceinline__ void slab_sum8(const float* p, long long slab_stride, int splits, float (&v)[8]) {
 #pragma unroll

@@ -122,14 +122,7 @@ __device__ __forceinline__ void regs_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(d)
-      : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
-  return *reinterpret_cast<float2*>(&d);
-}
-__device__ __forceinline__ float2 add_mul2(float2 a, float2 b, float2 f) {  // (a + b) * f
+__device__ __forceinline__ float2 add_mul_f32x2(float2 a, float2 b, float2 f) {  // (a + b) * f
   uint64_t d;
   asm("{\n\t.reg .b64 t;\n\t"
       "add.rn.f32x2 t, %1, %2;\n\t"
@@ -254,8 +247,8 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
       for (int g = 0; g < 16; ++g) {
         const float4 l = stat[g];
         const uint32_t* x = &rs[g / 8][(g % 8) * 4];
-        float2 a = fma2(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1])), sc2, make_float2(l.x, l.y));
-        float2 b = fma2(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3])), sc2, make_float2(l.z, l.w));
+        float2 a = fma_f32x2(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1])), sc2, make_float2(l.x, l.y));
+        float2 b = fma_f32x2(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3])), sc2, make_float2(l.z, l.w));
         pr[2 * g] = make_float2(fast_exp2(a.x), fast_exp2(a.y));
         pr[2 * g + 1] = make_float2(fast_exp2(b.x), fast_exp2(b.y));
       }
@@ -291,9 +284,9 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_consta
         for (int g = 0; g < 8; ++g) {
           const float4 dl = stat[32 + c * 8 + g];
           const uint32_t* x = &rs[0][g * 4];
-          const float2 a = add_mul2(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1])), make_float2(dl.x, dl.y),
+          const float2 a = add_mul_f32x2(make_float2(__uint_as_float(x[0]), __uint_as_float(x[1])), make_float2(dl.x, dl.y),
                                     pr[c * 16 + 2 * g]);
-          const float2 b = add_mul2(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3])), make_float2(dl.z, dl.w),
+          const float2 b = add_mul_f32x2(make_float2(__uint_as_float(x[2]), __uint_as_float(x[3])), make_float2(dl.z, dl.w),
                                     pr[c * 16 + 2 * g + 1]);
           dd[2 * g] = pack_bf16x2(a.x, a.y);
           dd[2 * g + 1] = pack_bf16x2(b.x, b.y);

@@ -440,8 +440,8 @@ extern "C" int sb_rope_kv_append(void* qkv, int row_stride, const float* slabs, 
   const long long cap = (long long)num_sms() * 8;
   if (blocks > cap) blocks = cap;
   return launch_chained(rope_kv_append_kernel, (unsigned)blocks, 256, 0, stream, (__nv_bfloat16*)qkv, row_stride, slabs,
-                        slab_stride, splits, (const __nv_bfloat16*)bias, rope_pos, pos_rows, sec0, sec1, cos_tab, sin_tab, seq_ids, cache_pos, block_table, max_blocks,
-                        (__nv_bfloat16*)cache, T, Hq, Hkv, D);
+                        slab_stride, splits, (const __nv_bfloat16*)bias, rope_pos, pos_rows, sec0, sec1, cos_tab, sin_tab,
+                        seq_ids, cache_pos, block_table, max_blocks, (__nv_bfloat16*)cache, T, Hq, Hkv, D);
 }
 
 extern "C" int sb_kv_copy_blocks(void* cache, const int* src, const int* dst, int n_pairs, long long block_elems,

@@ -26,7 +26,6 @@
 
 namespace sb {
 
-
 struct FmhaFwdParams {
   const int* tile_seq_start;  // [num_tiles] first token row of the tile's sequence
   const int* tile_seq_len;    // [num_tiles]
@@ -47,20 +46,6 @@ struct FwdSmem {
   static constexpr int kBarOff = kRingOff + kStages * kKvBytes;  // q[2], s_full[2], p_full[2], o_full[2], full[], empty[]
   static constexpr int kTotal = kBarOff + (8 + 2 * kStages) * 8 + 16;
 };
-
-__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(d)
-      : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&c)));
-  return *reinterpret_cast<float2*>(&d);
-}
-
-__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
-  return *reinterpret_cast<float2*>(&d);
-}
 
 // KV: keys of a tile; QT: query tiles; CTAS: blocks of an SM.
 // Four warps for the softmax of each query tile (thread = row), then one for TMA and the MMA issuer.

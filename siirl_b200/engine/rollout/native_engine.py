@@ -567,8 +567,8 @@ class RolloutEngine:
         use_cache = self.enable_prefix_caching and mm_inputs is None
         # Waiting prompts are prefilled while slots, blocks and tokens last before the next round of decode steps: a step
         # costs nearly the same for a few sequences as for all of them (96 prompts of a 0.5B policy, 33 tokens each: 80
-        # steps and 199 ms with decode rounds between the prefills, 32 steps and 108 ms without).  Chunked prefill keeps decoding in between (that
-        # is its purpose), and so do the ranks of a lock-step group, whose calls have to match.
+        # steps and 199 ms with decode rounds between the prefills, 32 steps and 108 ms without).  Chunked prefill keeps
+        # decoding in between (that is its purpose), and so do the ranks of a lock-step group, whose calls have to match.
         fill_first = not chunked and self.lockstep_group is None
         while group_any(bool(waiting) or any(s is not None for s in slots))[0]:
             # ---- prefill work of this iteration: continue started prompts, then admit new ones (all n samples of a

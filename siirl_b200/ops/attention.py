@@ -15,7 +15,6 @@ from . import lib as _lib
 from . import reference as ref
 
 
-_NUM_SMS = 148
 
 
 class SeqInfo:
@@ -85,7 +84,7 @@ def fwd_tile_rows(sequences: int, query_rows: int, hq: int, d: int) -> int:
     16 heads, one block an SM, 12 / 14; d = 64, 14 / 2: 256 x 64: 50 / 37, 128 x 128: 43 / 35, 64 x 160 30 / 31."""
     if query_rows <= 128 * sequences:
         return 128
-    if d == 128 and query_rows <= 384 * sequences and -(-query_rows // 256) * hq > _NUM_SMS:
+    if d == 128 and query_rows <= 384 * sequences and -(-query_rows // 256) * hq > _lib.NUM_SMS:
         return 128
     return 256
 
@@ -100,11 +99,11 @@ def bwd_head_splits(seqlens: Sequence[int], hq: int, hkv: int, causal: bool) -> 
     825, 845; 16 x 1000: 326, 301, 311, 326, 371."""
     rep = hq // hkv
     tiles = [(n + 127) // 128 for n in seqlens]
-    average = sum(t * (t + 1) // 2 if causal else t * t for t in tiles) * hq / _NUM_SMS
+    average = sum(t * (t + 1) // 2 if causal else t * t for t in tiles) * hq / _lib.NUM_SMS
     longest, blocks = max(tiles, default=0), sum(tiles) * hkv
 
     def steps(splits):
-        block, per_sm = -(-rep // splits) * longest, blocks * splits / _NUM_SMS
+        block, per_sm = -(-rep // splits) * longest, blocks * splits / _lib.NUM_SMS
         own = 5 * math.ceil(per_sm) + (per_sm if splits > 1 else 0)
         return max(block, average + block / max(1.0, per_sm) ** 2) + own
     return min(range(1, rep + 1), key=steps)

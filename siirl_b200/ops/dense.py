@@ -20,7 +20,6 @@ from . import lib as _lib
 from . import reference as ref
 
 EPI_BF16, EPI_F32_ACC, EPI_F32 = 0, 1, 2
-_NUM_SMS = 148
 EPI_BF16_T, EPI_F32_T = 4, 5        # transposed stores of the "weights in the A operand" form (see linear_skinny)
 
 
@@ -97,7 +96,7 @@ def _grad_splits(M: int, N: int, K: int) -> int:
 
     def cost(s):
         per = -(-nkb // s)
-        waves = -(-tiles * s // (_NUM_SMS // 2))
+        waves = -(-tiles * s // (_lib.NUM_SMS // 2))
         return waves * (0.4 * per + 3.0) + (4.0 + 2.4e-6 * s * M * N if s > 1 else 0.0)
     best = min(range(1, 9), key=cost)
     return best if best > 1 and nkb >= 4 * best and cost(best) < 0.8 * cost(1) else 1
@@ -176,8 +175,8 @@ def _skinny_splits(M: int, N: int, K: int) -> int:
     best, best_score = 1, -1.0
     for s in range(1, min(nkb // 4, 16) + 1):
         items = n_tiles * s
-        waves = (items + _NUM_SMS - 1) // _NUM_SMS
-        score = items / (waves * _NUM_SMS) - 0.01 * s       # wave efficiency, mild preference for fewer slabs
+        waves = (items + _lib.NUM_SMS - 1) // _lib.NUM_SMS
+        score = items / (waves * _lib.NUM_SMS) - 0.01 * s       # wave efficiency, mild preference for fewer slabs
         if score > best_score:
             best, best_score = s, score
     return best
@@ -191,8 +190,8 @@ def _best_splits(n_tiles: int, nkb: int) -> int:
     best, best_score = 1, -1.0
     for s in range(1, min(nkb // 4, 16) + 1):
         items = n_tiles * s
-        waves = (items + _NUM_SMS - 1) // _NUM_SMS
-        score = items / (waves * _NUM_SMS) - 0.01 * s
+        waves = (items + _lib.NUM_SMS - 1) // _lib.NUM_SMS
+        score = items / (waves * _lib.NUM_SMS) - 0.01 * s
         if score > best_score:
             best, best_score = s, score
     return best
@@ -239,7 +238,7 @@ def linear_skinny(x2: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.T
         return _linear_weights_as_a(x2, weight, bias)
     splits = _skinny_splits(M, N, K)
     if splits <= 1:
-        return gemm(x2, weight, bias=bias, tile_n=128 if N <= 128 * _NUM_SMS else 0)
+        return gemm(x2, weight, bias=bias, tile_n=128 if N <= 128 * _lib.NUM_SMS else 0)
     nkb = (K + 63) // 64
     per = (nkb + splits - 1) // splits
     eff = (nkb + per - 1) // per

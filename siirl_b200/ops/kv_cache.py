@@ -64,8 +64,9 @@ def rope_kv_append(qkv: torch.Tensor, rope_positions: torch.Tensor, cos_tab: tor
         if rows == 3:
             s0, s1 = mrope_section[0], mrope_section[0] + mrope_section[1]
         _lib.check(L.sb_rope_kv_append(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(slabs), ctypes.c_longlong(qkv.numel()),
-                                       slabs.shape[0] if slabs is not None else 0, _lib.ptr(bias), _lib.ptr(pos), rows, s0, s1, _lib.ptr(cos_tab),
-                                       _lib.ptr(sin_tab), _lib.ptr(seq_ids), _lib.ptr(cache_positions),
+                                       slabs.shape[0] if slabs is not None else 0, _lib.ptr(bias), _lib.ptr(pos), rows,
+                                       s0, s1, _lib.ptr(cos_tab), _lib.ptr(sin_tab), _lib.ptr(seq_ids),
+                                       _lib.ptr(cache_positions),
                                        _lib.ptr(block_table), block_table.shape[1], _lib.ptr(cache_layer),
                                        qkv.shape[0], n_heads, n_kv_heads, head_dim, _lib.stream()),
                    "sb_rope_kv_append")

@@ -14,6 +14,7 @@ from typing import Optional
 
 import torch
 
+NUM_SMS = 148       # of a B200: for rules on sizes that are evaluated without one
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libsiirl_b200.so"
 _lib: Optional["_CountingLib"] = None
 _status_words: dict[int, torch.Tensor] = {}

@@ -128,7 +128,8 @@ def fmha_bwd(qkv, out, lse, dout, info: SeqInfo, hq: int, hkv: int, d: int, caus
     turn = None
     if bwd_ordered(info.max_seqlen, d, causal):
         turn = torch.empty(hq * (T + 1), dtype=torch.int32, device=qkv.device)
-        dq_acc[info.total:].zero_()
+        if info.total < T:
+            dq_acc[info.total:].zero_()     # rows of no sequence
     ts, tl, t0, n = info.kv_tiles()
     rc = L.sb_fmha_bwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(delta), _lib.ptr(dq_acc),
                        _lib.ptr(dkv_acc), _lib.ptr(turn), _lib.ptr(dqkv), _lib.ptr(ts), _lib.ptr(tl), _lib.ptr(t0), n, T,

@@ -48,13 +48,15 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // rows costs a launch (2.9 us against some 0.3 us of memory time for 8 x 896) and a rounding.
 // Bound by memory.  All of a row's loads come before its first store, and the weights before the rows: the compiler may not
 // move them across a store by itself (9600 x 3584: 66 us with the stores of the sum in between, 46 us so).  Rows of up to
-// 2048 columns: eight blocks on an SM, as many as the grid has (9600 x 1024 with six: 17.7 us, with eight 14.7).
+// 2048 columns: eight blocks on an SM, as many as the grid has (9600 x 1024 with six: 17.7 us, with eight 14.7).  Partial sums
+// have at most 512 rows, for which four blocks are enough, and want the registers for loads in flight (8 x 896, 8 slabs:
+// 3.1 us with eight blocks, 2.3).
 // ---------------------------------------------------------------------------------------
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxChunks = 4;  // hidden <= 256 * 8 * 4 = 8192
 
 template <int CH, bool SLABS>
-__global__ void __launch_bounds__(kNormThreads, CH == 1 ? 8 : CH == 2 ? 4 : 2)
+__global__ void __launch_bounds__(kNormThreads, CH == 1 ? (SLABS ? 4 : 8) : CH == 2 && !SLABS ? 4 : 2)
 rmsnorm_fwd_kernel(const __nv_bfloat16* x, const float* slabs, long long slab_stride, int splits,
                    const __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* h_out,
                    float* rstd_out, int T, int H, float eps) {

@@ -50,7 +50,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // move them across a store by itself (9600 x 3584: 66 us with the stores of the sum in between, 46 us so).  Rows of up to
 // 2048 columns: eight blocks on an SM, as many as the grid has (9600 x 1024 with six: 17.7 us, with eight 14.7).  Partial sums
 // have at most 512 rows, for which four blocks are enough, and want the registers for loads in flight (8 x 896, 8 slabs:
-// 3.1 us with eight blocks, 2.3).
+// 3.1 us with eight blocks, 2.3 with three; 500 x 896, 3 slabs, 3.4 and 3.6, the rows beyond three blocks coming last).
 // ---------------------------------------------------------------------------------------
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxChunks = 4;  // hidden <= 256 * 8 * 4 = 8192
